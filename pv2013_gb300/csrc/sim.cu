@@ -1070,7 +1070,8 @@ lbm_status sim_create(const lbm_geometry* const* g, const lbm_sim_params* p, siz
     S->npl = p0.nodes_per_lane != 0 ? p0.nodes_per_lane : (S->store == ST_F64 ? 1 : 2);
     if (S->npl == 2 && S->store == ST_F64)
         return fail(LBM_ERR_ARG, "nodes_per_lane = 2 needs FP32 or 16-bit storage (FP64 runs one node per lane)");
-    if (S->wpb == 0) S->wpb = S->npl == 2 ? 1 : 4;
+    const bool default_wpb = S->wpb == 0;
+    if (default_wpb) S->wpb = S->npl == 2 ? 1 : 4;
     if (p0.piece_slots != 0 && p0.piece_slots != 8 && p0.piece_slots != 16 && p0.piece_slots != 32)
         return fail(LBM_ERR_ARG, "piece_slots must be 0, 8, 16 or 32 (got %d)", p0.piece_slots);
     // 8 slots (4 lanes) per piece: on the vascular tree 95 % of the slots
@@ -1138,6 +1139,12 @@ lbm_status sim_create(const lbm_geometry* const* g, const lbm_sim_params* p, siz
     S->N = node_off + kLatticeSlack;
     S->NF = out_off;
     S->nchunks = nch;
+    // FP64: a lattice that is one wave of warps (16 an SM) runs in one-warp
+    // blocks, which spread over the SMs to within one chunk (57 821-node vessel:
+    // 38.9 us a step against 42.7 with four-warp blocks); beyond that the
+    // staged ring's warps loop, and four-warp blocks are the better ones
+    // (151 680-node pipe: 92.2 us against 106.6)
+    if (default_wpb && S->store == ST_F64 && nch <= 152 * 16) S->wpb = 1;
     for (int k = 0; k < 3; ++k) S->nchunks2s[k] = nch2[k];
     S->nmask = nmask;
     S->nz = (int64_t)zall.size();

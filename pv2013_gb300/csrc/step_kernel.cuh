@@ -331,22 +331,104 @@ __device__ __forceinline__ void macro_ref(const T* f, T& rho, T& ux, T& uy, T& u
     }
 }
 
+// ---------------------------------------------------------------------------
+// FP64: the reference's results with fewer operations.  GB300 retires about 2
+// FP64 operations per clock and SM, which bounds every FP64 kernel here, so the
+// operation count is the time.
+
+// jx, jy, jz over rho, each the correctly rounded quotient.  One reciprocal
+// serves the three: with y = RN(1/rho), q = RN(j y) and the exact remainder
+// r = RN(j - q rho), RN(q + r y) is RN(j/rho) (Markstein 1990; Brisebarre, Muller
+// and Raina, "Accelerating correctly rounded floating-point division when the
+// divisor is known in advance", IEEE Trans. Computers 53(8), 2004) where
+// nothing under- or overflows: rho within 2^+-100 and j zero or within
+// 2^+-800 (remainders are multiples of |j| 2^-107).  Anything else, zero,
+// infinite and NaN operands too, takes the divisions.  A zero quotient may
+// come out +0 where the division gives -0.  Returns whether u is known finite.
+__device__ __forceinline__ bool div_in_range(double j) {
+    const uint32_t e = ((uint32_t)__double2hiint(j) >> 20) & 0x7ffu;
+    return e - (1023u - 800u) <= 1600u || j == 0.0;
+}
+__device__ __forceinline__ bool div3(double jx, double jy, double jz, double rho, double& ux, double& uy, double& uz) {
+    const uint32_t er = ((uint32_t)__double2hiint(rho) >> 20) & 0x7ffu;
+    const bool fast = er - (1023u - 100u) <= 200u && div_in_range(jx) && div_in_range(jy) && div_in_range(jz);
+    if (fast) {
+        const double y = 1.0 / rho;
+        const double qx = jx * y, qy = jy * y, qz = jz * y;
+        ux = __fma_rn(__fma_rn(-qx, rho, jx), y, qx);
+        uy = __fma_rn(__fma_rn(-qy, rho, jy), y, qy);
+        uz = __fma_rn(__fma_rn(-qz, rho, jz), y, qz);
+    } else {
+        ux = jx / rho;
+        uy = jy / rho;
+        uz = jz / rho;
+    }
+    return fast;
+}
+
+// sums of the populations in the reference's grouping (Simulation.cpp:32-79, :82-148)
+template <int Q, class T>
+__device__ __forceinline__ void moments_ref(const T* f, T& rho, T& jx, T& jy, T& jz) {
+    rho = f[0];
+#pragma unroll
+    for (int q = 1; q < Q; ++q) rho += f[q];
+    if constexpr (Q == 19) {
+        jx = (f[0] + f[6] + f[7] + f[8] + f[9]) - (f[1] + f[10] + f[11] + f[12] + f[13]);
+        jy = (f[2] + f[6] + f[10] + f[14] + f[15]) - (f[3] + f[7] + f[11] + f[16] + f[17]);
+        jz = (f[4] + f[8] + f[12] + f[14] + f[16]) - (f[5] + f[9] + f[13] + f[15] + f[17]);
+    } else {
+        jx = (f[1] + f[7] + f[8] + f[11] + f[13] + f[19] + f[21] + f[23] + f[25]) -
+             (f[2] + f[9] + f[10] + f[12] + f[14] + f[20] + f[22] + f[24] + f[26]);
+        jy = (f[3] + f[7] + f[9] + f[15] + f[16] + f[19] + f[21] + f[24] + f[26]) -
+             (f[4] + f[8] + f[10] + f[17] + f[18] + f[20] + f[22] + f[23] + f[25]);
+        jz = (f[5] + f[11] + f[12] + f[15] + f[17] + f[19] + f[22] + f[23] + f[26]) -
+             (f[6] + f[13] + f[14] + f[16] + f[18] + f[20] + f[21] + f[24] + f[25]);
+    }
+}
+
+// FP64 BGK collision, the reference's rounding on every population
+// (Simulation.cpp:21-179): f_eq = w rho (1 + 3 du + 9/2 du du - 3/2 u.u), f* =
+// omega f_eq + (1 - omega) f.  Left out is only what cannot change a bit: the
+// products of a velocity component with a zero c (a signed zero that is added
+// to du, gone in 1 + 3 du), and the second evaluation of du and 9/2 du du
+// for the opposite direction (du changes sign exactly).  D3Q19: 236
+// operations instead of 314.  A component that is not finite makes the
+// reference's every f_eq NaN (0 x inf); `one` carries that.
+template <int Q>
+__device__ __forceinline__ void collide64(double* f, double om) {
+    using L = Lat<Q>;
+    double rho, jx, jy, jz, ux, uy, uz;
+    moments_ref<Q, double>(f, rho, jx, jy, jz);
+    double one = 1.0;
+    if (!div3(jx, jy, jz, rho, ux, uy, uz)) one = 1.0 + (ux * 0.0 + uy * 0.0 + uz * 0.0);
+    const double usq15 = 3.0 / 2.0 * (ux * ux + uy * uy + uz * uz);
+    const double om1 = 1.0 - om;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const int o = L::opp(q);
+        const double wrho = L::w(q) * rho;
+        if (o == q) {
+            f[q] = om * (wrho * (one - usq15)) + om1 * f[q];
+        } else if (q < o) {
+            double du;
+            bool have = false;
+            if (L::cx(q)) { du = L::cx(q) > 0 ? ux : -ux; have = true; }
+            if (L::cy(q)) { du = have ? (L::cy(q) > 0 ? du + uy : du - uy) : (L::cy(q) > 0 ? uy : -uy); have = true; }
+            if (L::cz(q)) { du = have ? (L::cz(q) > 0 ? du + uz : du - uz) : (L::cz(q) > 0 ? uz : -uz); have = true; }
+            const double t3 = 3.0 * du, t45 = 9.0 / 2.0 * du * du;
+            f[q] = om * (wrho * (((one + t3) + t45) - usq15)) + om1 * f[q];
+            f[o] = om * (wrho * (((one - t3) + t45) - usq15)) + om1 * f[o];
+        }
+    }
+}
+
 // BGK collision.  F64: the reference's expressions.  FP32: shifted (and for
 // FP16 scaled) form with pairwise equilibrium.
 template <int Q, int S>
 __device__ __forceinline__ void collide(typename Work<S>::T* f, const InstParam& ip) {
     using L = Lat<Q>;
     if constexpr (S == ST_F64) {
-        double rho, ux, uy, uz;
-        macro_ref<Q, double>(f, rho, ux, uy, uz);
-        const double om = ip.omega;
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            const double du = ux * (double)L::cx(q) + uy * (double)L::cy(q) + uz * (double)L::cz(q);
-            const double usq = ux * ux + uy * uy + uz * uz;
-            const double feq = L::w(q) * rho * (1.0 + 3.0 * du + 9.0 / 2.0 * du * du - 3.0 / 2.0 * usq);
-            f[q] = om * feq + (1.0 - om) * f[q];
-        }
+        collide64<Q>(f, ip.omega);
     } else {
         constexpr float K = Work<S>::K;
         float drho = 0.f, jx = 0.f, jy = 0.f, jz = 0.f;
@@ -494,8 +576,10 @@ __device__ __forceinline__ void node_update(const StepArgs& a, int32_t zslot0, t
     }
 }
 
+// FP64 holds two registers a population and is bound by its arithmetic: 128
+// registers without spills (64 spilled 40 to 1060 bytes) and 16 warps an SM
 template <int Q, int S, int MODE, bool DRY, int RA>
-__global__ void __launch_bounds__(256, 4) k_step(StepArgs a, Partials part) {
+__global__ void __launch_bounds__(256, S == ST_F64 ? 2 : 4) k_step(StepArgs a, Partials part) {
     using L = Lat<Q>;
     using X = Ax<Q, RA>;
     using T = typename Work<S>::T;

@@ -32,7 +32,7 @@ static lbm_status launch_tma_one(const StepArgs& a, int32_t* err, int wpb, cudaS
     // one launch configuration per instantiation and block size: the grid is
     // the number of co-resident blocks (each warp loops over its chunks)
     static int cached_wpb = 0, cached_blocks = 0;
-    const size_t smem = (size_t)wpb * kStages * StageLayout<Q, S>::BYTES;
+    const size_t smem = (size_t)wpb * stage_count<S>() * StageLayout<Q, S>::BYTES;
     if (cached_wpb != wpb) {
         cudaError_t e = cudaFuncSetAttribute(k_step_tma<Q, S, MODE, RA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
