@@ -37,7 +37,8 @@ def collide_ref(f, Q, om):
 @pytest.mark.parametrize("staging", [0, 1])
 def test_collision_any_populations_bit_exact(tmp_path, Q, staging):
     c = cases.pipe(radius=7.0, length=33.0, ny=41, nxz=19)
-    sim = Simulation(c.geometry(), 0.83, (), Q=Q, precision="f64", pattern="aa", staging=staging)
+    sim = Simulation(c.geometry(), 0.83, (), Q=Q, precision="f64", pattern="aa", staging=staging,
+                     corrections=3)     # boundary nodes collide what their slots hold, like every other node
     path = str(tmp_path / "a.ckpt")
     sim.checkpoint(path)
     raw = np.fromfile(path, dtype=np.uint8)
@@ -50,7 +51,8 @@ def test_collision_any_populations_bit_exact(tmp_path, Q, staging):
         f[rng.integers(Q), k::40] = v            # one population of many nodes
         f[:, 20 + k::61] = v                     # every population of others
     f[:, 3::50] *= 1e-290
-    f[:, 4::50] *= 1e120
+    with np.errstate(over="ignore"):
+        f[:, 4::50] *= 1e120
     f[1:, 5::50] = 0.0                           # one population alone: j = rho
     old = f.copy()
     raw.tofile(path)
