@@ -24,7 +24,7 @@
 //      candidate lists.
 //   2. one warp per column, one lane per candidate: the z range in which the
 //      exact crossing test counts the candidate, as a parity mask over the
-//      column's points; one byte per point is written.
+//      column's points; one bit per point is written.
 // Because the ray is vertical, the xy inside test is independent of z, so
 // the split is exact.
 //
@@ -47,6 +47,7 @@
 #include <cstring>
 #include <vector>
 
+#include "bits.cuh"
 #include "device.cuh"
 #include "internal.h"
 #include "scan.cuh"
@@ -357,13 +358,13 @@ __device__ __forceinline__ bool cross_range(const VoxGrid& g, double inv_s, doub
 
 constexpr int kVoxWarps = 8;
 
-// One warp per column with candidates (the flags of the others are zero
+// One warp per column with candidates (the words of the others are zero
 // already), one lane per candidate.  Lane w holds the parity of points 32 w ..
 // 32 w + 31 and 32 (w + 32) .. (Nz <= 2048).
 __global__ void __launch_bounds__(kVoxWarps * 32)
 k_columns(VoxGrid g, double inv_s, const double* __restrict__ tris, const int64_t* __restrict__ colstart,
           const int32_t* __restrict__ pairs, const int32_t* __restrict__ global_list, int32_t nglobal,
-          uint8_t* __restrict__ flags) {
+          uint32_t* __restrict__ fluid) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t col = blockIdx.x * (int64_t)kVoxWarps + w;
     const int64_t ncol = (int64_t)g.Nx * g.Ny;
@@ -422,38 +423,54 @@ k_columns(VoxGrid g, double inv_s, const double* __restrict__ tris, const int64_
             }
         }
     }
-    // one byte per point
-    uint8_t* out = flags + col * (int64_t)g.Nz;
-    const int nb = (g.Nz + 31) / 32;
-    for (int b = 0; b < nb; ++b) {
-        const uint32_t word = __shfl_sync(0xffffffffu, b < 32 ? p0 : p1, b & 31);
-        if (word == 0u) continue;                      // (zero already)
-        const int z = 32 * b + lane;
-        if (z < g.Nz) out[z] = (uint8_t)((word >> lane) & 1u);
+    // (no candidate counts a point from Nz on, so the bits past the column are 0)
+    const int W = words_for(g.Nz);
+    uint32_t* out = fluid + col * W;
+    if (lane < W) out[lane] = p0;
+    if (lane + 32 < W) out[lane + 32] = p1;
+}
+
+// Boundary points, ComplexGeometry.cpp:509-556: fluid with a neighbour of the 26
+// that is not (outside the grid counts as not fluid, which makes the points on its
+// faces boundary points), one word a thread.
+__global__ void k_boundary(VoxGrid g, const uint32_t* __restrict__ fluid, uint32_t* __restrict__ isb) {
+    const int W = words_for(g.Nz);
+    const int64_t n = (int64_t)g.Nx * g.Ny * W;
+    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t f = fluid[p];
+        uint32_t r = 0;
+        if (f) {
+            const int w = (int)(p % W);
+            const int64_t ij = p / W;
+            const int j = (int)(ij % g.Ny), i = (int)(ij / g.Ny);
+            uint32_t all = f;                        // points whose neighbours are all fluid
+            if (i == 0 || i == g.Nx - 1 || j == 0 || j == g.Ny - 1) all = 0u;
+            for (int dx = -1; dx <= 1 && all; ++dx)
+                for (int dy = -1; dy <= 1; ++dy) {
+                    const uint32_t* c = fluid + ((int64_t)(i + dx) * g.Ny + (j + dy)) * W + w;
+                    const uint32_t m = c[0], lo = w > 0 ? c[-1] : 0u, hi = w + 1 < W ? c[1] : 0u;
+                    all &= m & ((m << 1) | (lo >> 31)) & ((m >> 1) | (hi << 31));
+                }
+            r = f & ~all;
+        }
+        isb[p] = r;
     }
 }
 
-// Boundary points: ComplexGeometry.cpp:509-556.
-__global__ void k_boundary(VoxGrid g, const uint8_t* __restrict__ flags, uint8_t* __restrict__ isb) {
-    const int64_t n = (int64_t)g.Nx * g.Ny * g.Nz;
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
-        uint8_t r = 0;
-        if (flags[p]) {
-            const int k = (int)(p % g.Nz);
-            const int64_t ij = p / g.Nz;
-            const int j = (int)(ij % g.Ny), i = (int)(ij / g.Ny);
-            bool b = (i == 0 || i == g.Nx - 1 || j == 0 || j == g.Ny - 1 || k == 0 || k == g.Nz - 1);
-            for (int dx = -1; dx <= 1 && !b; ++dx)
-                for (int dy = -1; dy <= 1 && !b; ++dy)
-                    for (int dz = -1; dz <= 1 && !b; ++dz) {
-                        const int a = i + dx, c = j + dy, e = k + dz;
-                        if (a >= 0 && a < g.Nx && c >= 0 && c < g.Ny && e >= 0 && e < g.Nz &&
-                            !flags[((int64_t)a * g.Ny + c) * g.Nz + e])
-                            b = true;
-                    }
-            r = b ? 1 : 0;
-        }
-        isb[p] = r;
+// x-major grid indices of the set bits, in order
+__global__ void k_bit_points(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ prefix, int64_t n, int W, int Nz,
+                             int64_t* __restrict__ out) {
+    for_each_bit(bits, prefix, n, [&](int64_t wi, uint32_t, int bit, uint32_t set, uint32_t rank) {
+        if (set) out[rank] = (wi / W) * Nz + (wi % W) * 32 + bit;
+    });
+}
+
+// bytes of grid points [first, first + n)
+__global__ void k_bit_bytes(const uint32_t* __restrict__ bits, int64_t first, int64_t n, int W, int Nz, uint8_t* __restrict__ out) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t p = first + i, col = p / Nz;
+        const int k = (int)(p - col * Nz);
+        out[i] = (uint8_t)((bits[col * W + (k >> 5)] >> (k & 31)) & 1u);
     }
 }
 
@@ -523,7 +540,7 @@ __global__ void k_gather_i64(const int64_t* __restrict__ src, const int64_t* __r
 struct lbm_geometry {
     lbm::VoxGrid grid;
     int dev = 0;
-    uint8_t* d_flags = nullptr;        // Nx*Ny*Nz
+    uint32_t* d_fluid = nullptr;       // fluid points, one bit each: words_for(Nz) words per column (x, y)
     int64_t* d_bidx = nullptr;         // boundary point grid indices
     uint64_t* d_bmask = nullptr;       // predicate mask per boundary point
     int64_t n_fluid = 0, n_boundary = 0;
@@ -598,7 +615,6 @@ static lbm_status geometry_build(lbm_geometry* G, const lbm_tri* tris, size_t nt
         g.Nx = d[0]; g.Ny = d[1]; g.Nz = d[2];
     }
     if (g.Nz > 2048) return fail(LBM_ERR_ARG, "Nz = %d exceeds the voxelizer's 2048-point column limit", g.Nz);
-    const int64_t npts = (int64_t)g.Nx * g.Ny * g.Nz;
     const int64_t ncol = (int64_t)g.Nx * g.Ny;
     for (size_t p = 0; p < npreds; ++p) {
         if (preds[p].list_id < 0 || preds[p].list_id > 63 || preds[p].axis < 0 || preds[p].axis > 2)
@@ -616,20 +632,22 @@ static lbm_status geometry_build(lbm_geometry* G, const lbm_tri* tris, size_t nt
     if (ntris) LBM_CUDA(cudaMemcpyAsync(d_tris.p, tris, sizeof(double) * 12 * ntris, cudaMemcpyHostToDevice, st));
     DBuf<int32_t> colcount, cursor, glist, nglob;
     DBuf<int64_t> colstart;
-    DBuf<uint8_t> flags;
+    DBuf<uint32_t> fluid;
     LBM_TRY(colcount.alloc(ncol, "column counts", st));
     LBM_TRY(cursor.alloc(ncol, "column cursors", st));
     LBM_TRY(colstart.alloc(ncol + 1, "column offsets", st));
     LBM_TRY(glist.alloc(ntris, "global triangle list", st));
     LBM_TRY(nglob.alloc(1, "global count", st));
-    LBM_TRY(flags.alloc(npts, "node-type field", st));
+    const int W = words_for(g.Nz);
+    const int64_t nwords = ncol * W;
+    LBM_TRY(fluid.alloc(nwords, "node-type field", st));
     LBM_CUDA(cudaEventRecord(e0, st));
     LBM_CUDA(cudaMemsetAsync(colcount.p, 0, sizeof(int32_t) * ncol, st));
     LBM_CUDA(cudaMemsetAsync(cursor.p, 0, sizeof(int32_t) * ncol, st));
     LBM_CUDA(cudaMemsetAsync(nglob.p, 0, sizeof(int32_t), st));
     const int TB = 128;
     const double inv_s = 1.0 / spacing;
-    LBM_CUDA(cudaMemsetAsync(flags.p, 0, npts, st));
+    LBM_CUDA(cudaMemsetAsync(fluid.p, 0, sizeof(uint32_t) * nwords, st));
     if (ntris) k_tri_count<<<(unsigned)((ntris + TB - 1) / TB), TB, 0, st>>>(g, inv_s, d_tris.p, (int64_t)ntris, colcount.p, glist.p, nglob.p);
     int64_t npairs = 0;
     LBM_TRY(scan::exclusive_scan(colcount.p, ncol, colstart.p, &npairs, st));
@@ -641,17 +659,21 @@ static lbm_status geometry_build(lbm_geometry* G, const lbm_tri* tris, size_t nt
     if (ntris) k_tri_fill<<<(unsigned)((ntris + TB - 1) / TB), TB, 0, st>>>(g, inv_s, d_tris.p, (int64_t)ntris, colstart.p, cursor.p, pairs.p);
     LBM_CUDA(cudaStreamSynchronize(st));
     k_columns<<<(unsigned)((ncol + kVoxWarps - 1) / kVoxWarps), kVoxWarps * 32, 0, st>>>(
-        g, inv_s, d_tris.p, colstart.p, pairs.p, glist.p, nglobal, flags.p);
+        g, inv_s, d_tris.p, colstart.p, pairs.p, glist.p, nglobal, fluid.p);
     LBM_CUDA(cudaGetLastError());
     LBM_CUDA(cudaEventRecord(e1, st));
 
     // boundary points and predicate lists
-    DBuf<uint8_t> isb;
-    LBM_TRY(isb.alloc(npts, "boundary flags", st));
-    k_boundary<<<g_blocks_for(npts, 256), 256, 0, st>>>(g, flags.p, isb.p);
-    LBM_TRY(scan::count_nonzero(flags.p, npts, &G->n_fluid, st));
+    DBuf<uint32_t> isb, rank;
+    LBM_TRY(isb.alloc(nwords, "boundary points", st));
+    LBM_TRY(rank.alloc(nwords, "boundary ranks", st));
+    k_boundary<<<g_blocks_for(nwords, 256), 256, 0, st>>>(g, fluid.p, isb.p);
+    LBM_TRY(scan::bit_ranks(fluid.p, nwords, nullptr, &G->n_fluid, st));
+    LBM_TRY(scan::bit_ranks(isb.p, nwords, rank.p, &G->n_boundary, st));
+    if (G->n_boundary > INT32_MAX) return fail(LBM_ERR_ARG, "more than 2^31 boundary points");
     int64_t* bidx = nullptr;
-    LBM_TRY(scan::compact(isb.p, npts, &bidx, &G->n_boundary, st));
+    LBM_TRY(dev_alloc(reinterpret_cast<void**>(&bidx), sizeof(int64_t) * std::max<int64_t>(G->n_boundary, 1), st, "boundary points"));
+    k_bit_points<<<g_blocks_for(nwords, 256), 256, 0, st>>>(isb.p, rank.p, nwords, W, g.Nz, bidx);
     G->d_bidx = bidx;
     DBuf<uint64_t> bmask;
     LBM_TRY(bmask.alloc(G->n_boundary, "boundary masks", st));
@@ -670,7 +692,7 @@ static lbm_status geometry_build(lbm_geometry* G, const lbm_tri* tris, size_t nt
     LBM_CUDA(cudaGetLastError());
     LBM_CUDA(cudaEventRecord(e2, st));
     G->d_bmask = bmask.release();
-    G->d_flags = flags.release();
+    G->d_fluid = fluid.release();
     G->n_lists = nl;
     G->list_sizes.assign(64, 0);
     {
@@ -765,7 +787,18 @@ lbm_status lbm_geometry_flags(const lbm_geometry* G, uint8_t* host_out, size_t c
     if (!G || !host_out) return fail(LBM_ERR_ARG, "lbm_geometry_flags: null argument");
     size_t n = (size_t)G->grid.Nx * G->grid.Ny * G->grid.Nz;
     if (cap < n) return fail(LBM_ERR_ARG, "lbm_geometry_flags: capacity %zu < %zu", cap, n);
-    LBM_CUDA(cudaMemcpy(host_out, G->d_flags, n, cudaMemcpyDeviceToHost));
+    // bits to bytes through a scratch of at most 32 MB
+    const size_t block = std::min<size_t>(n, size_t(32) << 20);
+    cudaStream_t st = 0;
+    DBuf<uint8_t> bytes;
+    LBM_TRY(bytes.alloc(block, "node-type bytes", st));
+    for (size_t at = 0; at < n; at += block) {
+        const size_t m = std::min(block, n - at);
+        k_bit_bytes<<<g_blocks_for((int64_t)m, 256), 256, 0, st>>>(G->d_fluid, (int64_t)at, (int64_t)m, words_for(G->grid.Nz),
+                                                                   G->grid.Nz, bytes.p);
+        LBM_CUDA(cudaGetLastError());
+        LBM_CUDA(cudaMemcpy(host_out + at, bytes.p, m, cudaMemcpyDeviceToHost));
+    }
     return LBM_OK;
 }
 
@@ -800,7 +833,7 @@ lbm_status lbm_geometry_list(const lbm_geometry* G, int32_t list, int64_t* host_
 void lbm_geometry_destroy(lbm_geometry* G) {
     if (!G) return;
     cudaDeviceSynchronize();               // pool memory is freed without an implicit wait
-    if (G->d_flags) cudaFree(G->d_flags);
+    if (G->d_fluid) cudaFree(G->d_fluid);
     if (G->d_bidx) cudaFree(G->d_bidx);
     if (G->d_bmask) cudaFree(G->d_bmask);
     delete G;
@@ -810,7 +843,7 @@ void lbm_geometry_destroy(lbm_geometry* G) {
 
 // accessors for the lattice builder (sim.cu)
 namespace lbm {
-const uint8_t* geometry_flags_dev(const lbm_geometry* g) { return g->d_flags; }
+const uint32_t* geometry_fluid_dev(const lbm_geometry* g) { return g->d_fluid; }
 const int64_t* geometry_bidx_dev(const lbm_geometry* g) { return g->d_bidx; }
 const uint64_t* geometry_bmask_dev(const lbm_geometry* g) { return g->d_bmask; }
 int64_t geometry_nboundary(const lbm_geometry* g) { return g->n_boundary; }

@@ -106,10 +106,10 @@ static __global__ void scan_totals(int64_t* __restrict__ tile_sum, int64_t ntile
     if (threadIdx.x == 0) *total = tot;
 }
 
-// Exclusive scan of counts into out (int64).
-template <class T>
+// Exclusive scan of counts into out.
+template <class T, class O>
 __global__ void tile_scan_write(const T* __restrict__ in, int64_t n, const int64_t* __restrict__ tile_off,
-                                int64_t* __restrict__ out) {
+                                O* __restrict__ out) {
     int64_t base = blockIdx.x * kTile + (int64_t)threadIdx.x * kItems;
     int64_t v[kItems];
     int64_t s = 0;
@@ -124,7 +124,7 @@ __global__ void tile_scan_write(const T* __restrict__ in, int64_t n, const int64
 #pragma unroll
     for (int i = 0; i < kItems; ++i) {
         int64_t idx = base + i;
-        if (idx < n) out[idx] = off;
+        if (idx < n) out[idx] = (O)off;
         off += v[i];
     }
 }
@@ -150,6 +150,44 @@ __global__ void tile_compact_write(const T* __restrict__ in, int64_t n, const in
 #pragma unroll
     for (int i = 0; i < kItems; ++i)
         if (bits & (1u << i)) out[off++] = base + i;
+}
+
+// Set bits of words: totals per tile, and the exclusive prefix of each word.
+__device__ __forceinline__ int load_words(const uint32_t* __restrict__ in, int64_t base, int64_t n, uint32_t* v) {
+    int s = 0;
+    if (base + kItems <= n) {
+#pragma unroll
+        for (int i = 0; i < kItems; i += 4) {
+            const uint4 q = *reinterpret_cast<const uint4*>(in + base + i);
+            v[i] = q.x; v[i + 1] = q.y; v[i + 2] = q.z; v[i + 3] = q.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < kItems; ++i) v[i] = base + i < n ? in[base + i] : 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) s += __popc(v[i]);
+    return s;
+}
+static __global__ void word_totals(const uint32_t* __restrict__ in, int64_t n, int64_t* __restrict__ tile_sum) {
+    uint32_t v[kItems];
+    const int s = load_words(in, blockIdx.x * kTile + (int64_t)threadIdx.x * kItems, n, v);
+    int64_t tot;
+    block_excl_scan(s, &tot);
+    if (threadIdx.x == 0) tile_sum[blockIdx.x] = tot;
+}
+static __global__ void word_prefix(const uint32_t* __restrict__ in, int64_t n, const int64_t* __restrict__ tile_off,
+                                   uint32_t* __restrict__ out) {
+    const int64_t base = blockIdx.x * kTile + (int64_t)threadIdx.x * kItems;
+    uint32_t v[kItems];
+    const int s = load_words(in, base, n, v);
+    int64_t tot;
+    uint32_t off = (uint32_t)(block_excl_scan(s, &tot) + tile_off[blockIdx.x]);
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) {
+        if (base + i < n) out[base + i] = off;
+        off += __popc(v[i]);
+    }
 }
 
 // Workspace for one scan of n elements.
@@ -180,18 +218,34 @@ inline void ws_free(Workspace& w) {
 }
 
 // Exclusive scan of n counts; *h_total receives the sum (synchronises stream).
-template <class T>
-lbm_status exclusive_scan(const T* d_in, int64_t n, int64_t* d_out, int64_t* h_total, cudaStream_t st) {
+template <class T, class O>
+lbm_status exclusive_scan(const T* d_in, int64_t n, O* d_out, int64_t* h_total, cudaStream_t st) {
     Workspace w;
     lbm_status s = ws_alloc(w, n, st);
     if (s != LBM_OK) return s;
     tile_totals<T><<<(unsigned)w.ntiles, kThreads, 0, st>>>(d_in, n, w.tiles, false);
     scan_totals<<<1, kThreads, 0, st>>>(w.tiles, w.ntiles, w.total);
-    tile_scan_write<T><<<(unsigned)w.ntiles, kThreads, 0, st>>>(d_in, n, w.tiles, d_out);
+    tile_scan_write<T, O><<<(unsigned)w.ntiles, kThreads, 0, st>>>(d_in, n, w.tiles, d_out);
     cudaError_t e = cudaMemcpyAsync(h_total, w.total, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     ws_free(w);
     if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "exclusive_scan: %s", cudaGetErrorString(e));
+    return LBM_OK;
+}
+
+// Set bits of n words (synchronises), and their exclusive prefix per word where
+// d_prefix is not null (valid when the total fits 32 bits).
+inline lbm_status bit_ranks(const uint32_t* d_in, int64_t n, uint32_t* d_prefix, int64_t* h_total, cudaStream_t st) {
+    Workspace w;
+    lbm_status s = ws_alloc(w, n, st);
+    if (s != LBM_OK) return s;
+    word_totals<<<(unsigned)w.ntiles, kThreads, 0, st>>>(d_in, n, w.tiles);
+    scan_totals<<<1, kThreads, 0, st>>>(w.tiles, w.ntiles, w.total);
+    if (d_prefix) word_prefix<<<(unsigned)w.ntiles, kThreads, 0, st>>>(d_in, n, w.tiles, d_prefix);
+    cudaError_t e = cudaMemcpyAsync(h_total, w.total, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    ws_free(w);
+    if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "bit_ranks: %s", cudaGetErrorString(e));
     return LBM_OK;
 }
 

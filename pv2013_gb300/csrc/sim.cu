@@ -27,6 +27,7 @@
 #include <string>
 #include <vector>
 
+#include "bits.cuh"
 #include "device.cuh"
 #include "internal.h"
 #include "scan.cuh"
@@ -36,7 +37,7 @@
 
 namespace lbm {
 // geometry accessors (geometry.cu)
-const uint8_t* geometry_flags_dev(const lbm_geometry* g);
+const uint32_t* geometry_fluid_dev(const lbm_geometry* g);
 const int64_t* geometry_bidx_dev(const lbm_geometry* g);
 const uint64_t* geometry_bmask_dev(const lbm_geometry* g);
 int64_t geometry_nboundary(const lbm_geometry* g);
@@ -123,147 +124,140 @@ int blocks_for(int64_t n, int threads) {
 // --------------------------------------------------------------------------
 // set-up kernels
 
-__global__ void k_scatter_ids(const int64_t* __restrict__ node_grid, int64_t n, int32_t* __restrict__ node_of_point) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        node_of_point[node_grid[i]] = (int32_t)i;
-}
-
-// Grid permutation for the run axis.  Permuted layout: index (a*Nb + b)*Nr + r
-// with r the run axis; for run axis z it is the x-major layout itself, for
-// run axis y it is (x*Nz + z)*Ny + y.
+// Grid axes by role for a run axis: columns (a, b), levels r.  Run axis z: (x, y)
+// and z; run axis y: (x, z) and y.
 struct Perm {
     int ra;             // 1 (y) or 2 (z)
     int Nx, Ny, Nz;
     __host__ __device__ int Na() const { return Nx; }
     __host__ __device__ int Nb() const { return ra == 2 ? Ny : Nz; }
     __host__ __device__ int Nr() const { return ra == 2 ? Nz : Ny; }
-    __host__ __device__ int64_t to_perm(int64_t o) const {
-        if (ra == 2) return o;
-        const int64_t k = o % Nz, t = o / Nz, j = t % Ny, i = t / Ny;
-        return (i * Nz + k) * Ny + j;
-    }
-    __host__ __device__ int64_t to_orig(int64_t p) const {
-        if (ra == 2) return p;
-        const int64_t j = p % Ny, t = p / Ny, k = t % Nz, i = t / Nz;
-        return (i * Ny + j) * Nz + k;
-    }
 };
 
-__global__ void k_permute_flags(const uint8_t* __restrict__ in, Perm P, uint8_t* __restrict__ out) {
-    const int64_t n = (int64_t)P.Nx * P.Ny * P.Nz;
-    for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x)
-        out[P.to_perm(o)] = in[o];
+// Fluid bits along z (word wz of column (x, y)) to fluid bits along y (word wy of
+// column (x, z)): 32x32 blocks, one warp each.
+__global__ void k_transpose_bits(const uint32_t* __restrict__ in, int Nx, int Ny, int Nz, uint32_t* __restrict__ out) {
+    const int lane = threadIdx.x & 31, Wz = words_for(Nz), Wy = words_for(Ny);
+    const int64_t n = (int64_t)Nx * Wy * Wz;
+    for (int64_t v = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; v < n; v += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+        const int wz = (int)(v % Wz), wy = (int)(v / Wz % Wy), x = (int)(v / Wz / Wy);
+        const int y = 32 * wy + lane, z = 32 * wz + lane;
+        const uint32_t w = transpose32(y < Ny ? in[((int64_t)x * Ny + y) * Wz + wz] : 0u);
+        if (z < Nz) out[((int64_t)x * Nz + z) * Wy + wy] = w;
+    }
 }
 
-// Node types on the padded permuted grid (one extra cell on every side):
-// 2 fluid, 1 ghost (not fluid, a fluid point among its 26 neighbours), 0 none.
+// The grid padded by one cell on every side, in bits along the run axis: padded
+// column (a, b) has words_for(Pr) words, level r at bit r.  Fluid bits are kept
+// unpadded (level r is bit r - 1 of unpadded column (a - 1, b - 1)).
 struct Pad {
-    int Na, Nb, Nr;                       // unpadded permuted dims
-    __host__ __device__ int64_t Pa() const { return Na + 2; }
-    __host__ __device__ int64_t Pb() const { return Nb + 2; }
+    int Na, Nb, Nr;                       // unpadded dims
+    __host__ __device__ int Pb() const { return Nb + 2; }
     // padded run-axis length, rounded up to even (node ids keep the parity of
     // their level, which needs every column to end at an odd level)
-    __host__ __device__ int64_t Pr() const { return (Nr + 3) & ~int64_t(1); }
-    __host__ __device__ int64_t cells() const { return Pa() * Pb() * Pr(); }
-    __host__ __device__ int64_t cell(int64_t a, int64_t b, int64_t r) const { return (a * Pb() + b) * Pr() + r; }
+    __host__ __device__ int Pr() const { return (Nr + 3) & ~1; }
+    __host__ __device__ int W() const { return words_for(Pr()); }
+    __host__ __device__ int64_t words() const { return (int64_t)(Na + 2) * Pb() * W(); }
+    __host__ __device__ int64_t col(int a, int b) const { return (int64_t)a * Pb() + b; }
+};
+struct Lattice {
+    Pad D;
+    const uint32_t* fluid;    // unpadded columns (a, b), words_for(Nr) words
+    const uint32_t* nodes;    // padded columns: fluid and ghost points
+    const uint32_t* rank;     // node ids before each word of nodes
+    // word w of padded column (a, b): its fluid levels
+    __device__ uint32_t fluid_word(int a, int b, int w) const {
+        if (a < 1 || a > D.Na || b < 1 || b > D.Nb) return 0u;
+        const int Wu = words_for(D.Nr);
+        const uint32_t* c = fluid + ((int64_t)(a - 1) * D.Nb + (b - 1)) * Wu;
+        const uint32_t m = w < Wu ? c[w] : 0u, lo = w > 0 && w - 1 < Wu ? c[w - 1] : 0u;
+        return (m << 1) | (lo >> 31);
+    }
+    __device__ bool is_fluid(int a, int b, int r) const {
+        if (a < 1 || a > D.Na || b < 1 || b > D.Nb || r < 1 || r > D.Nr) return false;
+        return (fluid[((int64_t)(a - 1) * D.Nb + (b - 1)) * words_for(D.Nr) + ((r - 1) >> 5)] >> ((r - 1) & 31)) & 1u;
+    }
+    // node id of a padded point, -1 where there is none
+    __device__ int32_t id(int a, int b, int r) const {
+        const int64_t wi = D.col(a, b) * D.W() + (r >> 5);
+        const uint32_t w = nodes[wi];
+        if (!((w >> (r & 31)) & 1u)) return -1;
+        return (int32_t)(rank[wi] + __popc(w & ((1u << (r & 31)) - 1u)));
+    }
 };
 
-// Node types by separable dilation: the 3x3x3 neighbourhood test as three
-// 3-point passes (run axis, b, a), one thread per cell with the coordinates
-// taken from the launch grid.
-__global__ void k_dil_r(const uint8_t* __restrict__ pflags, Pad D, uint8_t* __restrict__ t1) {
-    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t b = blockIdx.y, a = blockIdx.z;
-    if (r >= D.Pr()) return;
-    uint8_t v = 0;
-    if (a >= 1 && a <= D.Na && b >= 1 && b <= D.Nb) {
-        const uint8_t* col = pflags + ((a - 1) * D.Nb + (b - 1)) * (int64_t)D.Nr;
-        for (int64_t rr = r - 1; rr <= r + 1; ++rr)
-            if (rr >= 1 && rr <= D.Nr && col[rr - 1]) v = 1;
-    }
-    t1[D.cell(a, b, r)] = v;
-}
-__global__ void k_dil_b(const uint8_t* __restrict__ t1, Pad D, uint8_t* __restrict__ t2) {
-    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t b = blockIdx.y, a = blockIdx.z;
-    if (r >= D.Pr()) return;
-    uint8_t v = 0;
-    for (int64_t bb = b - 1; bb <= b + 1; ++bb)
-        if (bb >= 0 && bb < D.Pb()) v |= t1[D.cell(a, bb, r)];
-    t2[D.cell(a, b, r)] = v;
-}
-__global__ void k_dil_a(const uint8_t* __restrict__ t2, const uint8_t* __restrict__ pflags, Pad D,
-                        uint8_t* __restrict__ type) {
-    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t b = blockIdx.y, a = blockIdx.z;
-    if (r >= D.Pr()) return;
-    uint8_t v = 0;
-    for (int64_t aa = a - 1; aa <= a + 1; ++aa)
-        if (aa >= 0 && aa < D.Pa()) v |= t2[D.cell(aa, b, r)];
-    const bool fluid = a >= 1 && a <= D.Na && b >= 1 && b <= D.Nb && r >= 1 && r <= D.Nr &&
-                       pflags[((a - 1) * D.Nb + (b - 1)) * (int64_t)D.Nr + (r - 1)] != 0;
-    type[D.cell(a, b, r)] = fluid ? 2 : (v ? 1 : 0);
-}
-
-// type of every padded cell (2 fluid, 1 ghost, 0 none); scratch: one more
-// byte per cell
-lbm_status compute_types(const uint8_t* pflags, const Pad& D, uint8_t* type, cudaStream_t st) {
-    DBuf<uint8_t> tmp;
-    LBM_TRY(tmp.alloc(D.cells(), "node type scratch", st));
-    const dim3 grid((unsigned)((D.Pr() + 255) / 256), (unsigned)D.Pb(), (unsigned)D.Pa());
-    k_dil_r<<<grid, 256, 0, st>>>(pflags, D, type);
-    k_dil_b<<<grid, 256, 0, st>>>(type, D, tmp.p);
-    k_dil_a<<<grid, 256, 0, st>>>(tmp.p, pflags, D, type);
-    LBM_CUDA(cudaGetLastError());
-    LBM_CUDA(cudaStreamSynchronize(st));   // the scratch is freed on return
-    return LBM_OK;
-}
-
-// Extra ghost nodes so that every node id has the parity of its level: one
-// below every segment of consecutive nodes that starts at an odd level and one
-// above every segment that ends at an even level.  Then every segment starts
-// at an even level and has even length, so ids (assigned in cell order) keep
-// id = level (mod 2).  Changing a cell in place never changes another cell's
-// test.
-__global__ void k_parity_ghosts(Pad D, uint8_t* __restrict__ type) {
-    const int64_t n = D.cells();
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
-        if (type[c]) continue;
-        const int64_t r = c % D.Pr();
-        if ((r & 1) == 0 ? (r + 1 < D.Pr() && type[c + 1]) : (type[c - 1] != 0)) type[c] = 1;
+// Nodes: every point within one cell of a fluid point, and extra ghosts so that
+// every node id has the parity of its level: one below every segment of
+// consecutive nodes that starts at an odd level and one above every segment that
+// ends at an even level, that is, both levels of every pair (2k, 2k + 1) that
+// holds a node.  Then every segment starts at an even level and has even length,
+// so ids (assigned in cell order) keep id = level (mod 2).
+__global__ void k_node_bits(Lattice A, uint32_t* __restrict__ out) {
+    const Pad& D = A.D;
+    const int W = D.W(), Wu = words_for(D.Nr);
+    const int64_t n = D.words();
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+        const int w = (int)(v % W);
+        const int64_t c = v / W;
+        const int b = (int)(c % D.Pb()), a = (int)(c / D.Pb());
+        uint32_t m = 0, lo = 0;               // unpadded words w and w - 1 over the nine columns
+        for (int aa = max(a - 1, 1); aa <= min(a + 1, D.Na); ++aa)
+            for (int bb = max(b - 1, 1); bb <= min(b + 1, D.Nb); ++bb) {
+                const uint32_t* u = A.fluid + ((int64_t)(aa - 1) * D.Nb + (bb - 1)) * Wu;
+                if (w < Wu) m |= u[w];
+                if (w > 0 && w - 1 < Wu) lo |= u[w - 1];
+            }
+        // levels r - 1, r, r + 1 are unpadded bits r - 2, r - 1, r
+        const uint32_t d = m | (m << 1) | (lo >> 31) | (m << 2) | (lo >> 30);
+        out[v] = d | ((d & 0x55555555u) << 1) | ((d & 0xaaaaaaaau) >> 1);
     }
 }
 
-// out_pos of every node: x-major rank of its fluid point (ghosts: -1)
-__global__ void k_out_pos(const int64_t* __restrict__ node_cell, int64_t n, const uint8_t* __restrict__ type, Pad D,
-                          Perm P, const int32_t* __restrict__ rank_of_point, int64_t out_off, int32_t* __restrict__ pos) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t c = node_cell[i];
-        if (type[c] != 2) { pos[i] = -1; continue; }
-        const int64_t r = c % D.Pr(), t = c / D.Pr();
-        const int64_t b = t % D.Pb(), a = t / D.Pb();
-        const int64_t p = ((a - 1) * D.Nb + (b - 1)) * D.Nr + (r - 1);
-        pos[i] = (int32_t)(out_off + rank_of_point[P.to_orig(p)]);
-    }
+// role (-1 ghost, 0 fluid; k_roles sets the boundary nodes) and output position
+// (x-major rank of the fluid point, -1 for ghosts) of every node
+__global__ void k_nodes(Lattice A, Perm P, const uint32_t* __restrict__ zfluid, const uint32_t* __restrict__ zrank,
+                        int64_t out_off, int8_t* __restrict__ role, int32_t* __restrict__ pos) {
+    const int W = A.D.W(), Wz = words_for(P.Nz);
+    for_each_bit(A.nodes, A.rank, A.D.words(), [&](int64_t wi, uint32_t, int bit, uint32_t set, uint32_t id) {
+        const int w = (int)(wi % W);
+        const int64_t c = wi / W;
+        const int b = (int)(c % A.D.Pb()), a = (int)(c / A.D.Pb());
+        const bool fl = (A.fluid_word(a, b, w) >> bit) & 1u;
+        if (!set) return;
+        int32_t o = -1;
+        if (fl) {
+            const int r = 32 * w + bit, y = P.ra == 2 ? b - 1 : r - 1, z = P.ra == 2 ? r - 1 : b - 1;
+            const int64_t zw = ((int64_t)(a - 1) * P.Ny + y) * Wz + (z >> 5);
+            o = (int32_t)(out_off + zrank[zw] + __popc(zfluid[zw] & ((1u << (z & 31)) - 1u)));
+        }
+        role[id] = fl ? 0 : -1;
+        pos[id] = o;
+    });
+}
+
+// x-major grid index of every fluid point, in x-major order
+__global__ void k_points(const uint32_t* __restrict__ zfluid, const uint32_t* __restrict__ zrank, int64_t n, int Wz, int Nz,
+                         int64_t* __restrict__ out) {
+    for_each_bit(zfluid, zrank, n, [&](int64_t wi, uint32_t, int bit, uint32_t set, uint32_t rank) {
+        if (set) out[rank] = (wi / Wz) * Nz + (wi % Wz) * 32 + bit;
+    });
 }
 
 // role per node: -1 ghost, 0 interior, 1 wall, 2+l first matching predicate list l
-__global__ void k_roles_fluid(const int64_t* __restrict__ node_cell, int64_t n, const uint8_t* __restrict__ type,
-                              int8_t* __restrict__ role) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        role[i] = type[node_cell[i]] == 2 ? 0 : -1;
-}
-
-__global__ void k_roles(const int64_t* __restrict__ bidx, const uint64_t* __restrict__ bmask, int64_t nb, Perm P, Pad D,
-                        const int32_t* __restrict__ node_of_cell, int8_t* __restrict__ role) {
+__global__ void k_roles(const int64_t* __restrict__ bidx, const uint64_t* __restrict__ bmask, int64_t nb, Lattice A, Perm P,
+                        int8_t* __restrict__ role) {
     for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < nb; b += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t p = P.to_perm(bidx[b]);
-        const int64_t r = p % D.Nr, t = p / D.Nr;
-        const int64_t bb = t % D.Nb, a = t / D.Nb;
-        const int32_t n = node_of_cell[D.cell(a + 1, bb + 1, r + 1)];
+        const int64_t p = bidx[b], c = p / P.Nz;
+        const int z = (int)(p - c * P.Nz), y = (int)(c % P.Ny), x = (int)(c / P.Ny);
+        const int32_t n = P.ra == 2 ? A.id(x + 1, y + 1, z + 1) : A.id(x + 1, z + 1, y + 1);
         const uint64_t m = bmask[b];
         role[n] = m ? (int8_t)(2 + __ffsll((long long)m) - 1) : (int8_t)1;
     }
+}
+
+__global__ void k_boundary_flag(const int8_t* __restrict__ role, int64_t n, uint8_t* __restrict__ out) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = role[i] >= 1 ? 1 : 0;
 }
 
 __global__ void k_zflag(const int8_t* __restrict__ role, int64_t n, uint64_t zlists, uint8_t* __restrict__ z) {
@@ -281,30 +275,34 @@ __global__ void k_gather_role(const int64_t* __restrict__ ids, int64_t n, const 
     }
 }
 
-// per padded column (a, b): chunks (runs of fluid cells, <= 32) and boundary lanes
-__global__ void k_col_count(const uint8_t* __restrict__ type, const int32_t* __restrict__ node_of_cell,
-                            const int8_t* __restrict__ role, Pad D, int32_t* __restrict__ nchunk,
-                            int32_t* __restrict__ nbound) {
-    const int64_t ncol = (int64_t)D.Na * D.Nb;
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncol; c += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t a = c / D.Nb + 1, b = c % D.Nb + 1;
-        const int64_t base = D.cell(a, b, 0);
-        int32_t nc = 0, nbd = 0;
-        int run = 0;
-        for (int64_t r = 0; r <= D.Pr(); ++r) {
-            const bool fl = r < D.Pr() && type[base + r] == 2;
-            if (fl) {
-                ++run;
-                if (role[node_of_cell[base + r]] >= 1) ++nbd;
+// Calls fn(first level, last level) for every run of consecutive fluid levels of
+// padded column (a, b); stops when fn returns false.
+template <class F>
+__device__ __forceinline__ void for_each_run(const Lattice& A, int a, int b, F fn) {
+    const int W = A.D.W();
+    int rf = -1;
+    for (int w = 0; w < W; ++w) {
+        uint32_t v = A.fluid_word(a, b, w);          // bits below the next run's start are 0; of an open run, 1
+        if (rf >= 0 && v == 0xffffffffu) continue;
+        for (;;) {
+            if (rf < 0) {
+                if (v == 0u) break;
+                rf = 32 * w + __ffs(v) - 1;
+                v |= (1u << (rf & 31)) - 1u;
             }
-            if (!fl || run == 32) {
-                if (run > 0) ++nc;
-                run = 0;
-            }
+            const uint32_t off = ~v;
+            if (off == 0u) break;
+            const int e = __ffs(off) - 1;
+            if (!fn(rf, 32 * w + e - 1)) return;
+            rf = -1;
+            v &= ~((1u << e) - 1u);
         }
-        nchunk[c] = nc;
-        nbound[c] = nbd;
     }
+}
+// pieces of `piece` slots of a run, widened to whole pairs of levels when `pairs`
+__device__ __forceinline__ int run_pieces(int rf, int re, int piece, bool pairs) {
+    const int lo = pairs ? rf & ~1 : rf, hi = pairs ? re | 1 : re;
+    return (hi - lo + piece) / piece;
 }
 
 struct Vel {
@@ -312,21 +310,53 @@ struct Vel {
     int Q;
 };
 
+// missing-population mask of every boundary node, in node order
+__global__ void k_masks(Lattice A, Vel V, const int8_t* __restrict__ role, const uint32_t* __restrict__ brank,
+                        uint32_t* __restrict__ mmask) {
+    const int W = A.D.W();
+    for_each_bit(A.nodes, A.rank, A.D.words(), [&](int64_t wi, uint32_t, int bit, uint32_t set, uint32_t id) {
+        if (!set || role[id] < 1) return;
+        const int r = (int)(wi % W) * 32 + bit;
+        const int64_t c = wi / W;
+        const int b = (int)(c % A.D.Pb()), a = (int)(c / A.D.Pb());
+        uint32_t m = 0;
+        for (int q = 0; q < V.Q; ++q)
+            if (!A.is_fluid(a - V.a[q], b - V.b[q], r - V.r[q])) m |= 1u << q;
+        mmask[brank[id]] = m;
+    });
+}
+
+// per column: chunks (runs cut every 32 nodes) and paired pieces of 8, 16, 32 slots
+struct PieceCounts {
+    int32_t* n[4];
+};
+__global__ void k_piece_counts(Lattice A, int sizes, PieceCounts C) {
+    const int64_t ncol = (int64_t)A.D.Na * A.D.Nb;
+    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncol; c += (int64_t)gridDim.x * blockDim.x) {
+        int32_t n[4] = {0, 0, 0, 0};
+        for_each_run(A, (int)(c / A.D.Nb) + 1, (int)(c % A.D.Nb) + 1, [&](int rf, int re) {
+            n[0] += run_pieces(rf, re, 32, false);
+            n[1] += run_pieces(rf, re, 8, true);
+            n[2] += run_pieces(rf, re, 16, true);
+            n[3] += run_pieces(rf, re, 32, true);
+            return true;
+        });
+        for (int k = 0; k < sizes; ++k) C.n[k][c] = n[k];
+    }
+}
+
 struct FillArgs {
-    const uint8_t* type;
-    const int32_t* node_of_cell;
+    Lattice A;
     const int8_t* role;
-    Pad D;
-    Vel V;
-    const int64_t* chunk_off;     // per column
-    const int64_t* mslot_off;     // per column
+    const uint32_t* brank;        // boundary nodes before each node
+    const int64_t* off;           // pieces before each column
+    int64_t pieces;
     const int64_t* znodes;        // sorted local ids of Zou-He nodes
     int64_t nz;
     int64_t node_off, zslot_off, mslot_base;
     int32_t inst;
-    int32_t piece;                // node slots per paired chunk piece (k_col_fill2)
+    int32_t piece;                // node slots per piece
     Chunk* chunks;
-    uint32_t* mmask;
     int32_t* err;
 };
 
@@ -339,144 +369,69 @@ __device__ int64_t lower_bound_i64(const int64_t* a, int64_t n, int64_t v) {
     return lo;
 }
 
-__global__ void k_col_fill(FillArgs A) {
+// One thread per piece: its column by bisection of the offsets, its run from the
+// column's bits.  PAIR: each fluid run [rf, re] widened to whole pairs [rf & ~1,
+// re | 1] (the added slots are ghost nodes) and cut every `piece` slots;
+// otherwise runs cut every `piece` nodes.  (One thread per column, walking its
+// levels byte by byte, took 3.8 ms for the tree's chunks and 2.5 ms for each paired
+// table; 60 to 128 us a table now.)
+template <bool PAIR>
+__global__ void __launch_bounds__(128) k_fill_pieces(FillArgs F) {
+    const Lattice& A = F.A;
     const Pad& D = A.D;
     const int64_t ncol = (int64_t)D.Na * D.Nb;
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncol; c += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t a = c / D.Nb + 1, b = c % D.Nb + 1;
-        const int64_t base = D.cell(a, b, 0);
-        int64_t out = A.chunk_off[c];
-        int64_t ms = A.mslot_off[c];
-        int run = 0;
-        int64_t r0 = 0;
-        for (int64_t r = 0; r <= D.Pr(); ++r) {
-            const bool fl = r < D.Pr() && A.type[base + r] == 2;
-            if (fl) { if (run == 0) r0 = r; ++run; }
-            if (!fl || run == 32) {
-                if (run > 0) {
-                    Chunk ch;
-                    const int32_t n0 = A.node_of_cell[base + r0];
-                    ch.n0 = (int32_t)(A.node_off + n0);
-                    ch.len_inst = (uint32_t)run | ((uint32_t)A.inst << 8);
-                    ch.wmask = ch.zmask = ch.bmask = 0;
-                    ch.vmask = run == 32 ? 0xffffffffu : (1u << run) - 1u;
-                    ch.mslot0 = (int32_t)(A.mslot_base + ms);
-                    for (int t = 0; t < run; ++t) {
-                        const int ro = A.role[n0 + t];
-                        if (ro == 1) ch.wmask |= 1u << t;
-                        if (ro >= 1) {
-                            ch.bmask |= 1u << t;
-                            uint32_t m = 0;
-                            for (int q = 0; q < A.V.Q; ++q) {
-                                const int64_t sc = D.cell(a - A.V.a[q], b - A.V.b[q], r0 + t - A.V.r[q]);
-                                if (A.type[sc] != 2) m |= 1u << q;
-                            }
-                            A.mmask[ms++] = m;
-                        }
-                    }
-                    const int64_t zfirst = lower_bound_i64(A.znodes, A.nz, n0);
-                    ch.zslot0 = (int32_t)(A.zslot_off + zfirst);
-                    for (int64_t zz = zfirst; zz < A.nz && A.znodes[zz] < n0 + run; ++zz)
-                        ch.zmask |= 1u << (int)(A.znodes[zz] - n0);
-                    for (int da = -1; da <= 1; ++da)
-                        for (int db = -1; db <= 1; ++db) {
-                            if (da == 0 && db == 0) continue;
-                            const int32_t k = A.node_of_cell[D.cell(a + da, b + db, r0 - 1)];
-                            // every level r0-1 .. r0+run of a neighbour column is a node
-                            // with consecutive ids (ghost layer); checked at both ends
-                            const int32_t k2 = A.node_of_cell[D.cell(a + da, b + db, r0 + run)];
-                            if (k < 0 || k2 != k + run + 1) atomicOr(A.err, 1);
-                            ch.K[col8(da, db)] = (int32_t)(A.node_off + (k < 0 ? 0 : k));
-                        }
-                    if (n0 < 1 || A.node_of_cell[base + r0 - 1] != n0 - 1 ||
-                        A.node_of_cell[base + r0 + run] != n0 + run)
-                        atomicOr(A.err, 1);
-                    A.chunks[out++] = ch;
-                }
-                run = 0;
-            }
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < F.pieces; i += (int64_t)gridDim.x * blockDim.x) {
+        int64_t c = 0, hi = ncol - 1;                // last column with off <= i (empty columns share its successor's)
+        while (c < hi) {
+            const int64_t mid = (c + hi + 1) >> 1;
+            if (F.off[mid] <= i) c = mid; else hi = mid - 1;
         }
-    }
-}
-
-// Paired chunks: each fluid run [rf, re] of a column widened to whole pairs
-// [rf & ~1, re | 1] (the added slots are ghost nodes) and cut every `piece`
-// slots (8, 16 or 32).
-__global__ void k_col_count2(const uint8_t* __restrict__ type, Pad D, int piece, int32_t* __restrict__ nchunk) {
-    const int64_t ncol = (int64_t)D.Na * D.Nb;
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncol; c += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t a = c / D.Nb + 1, b = c % D.Nb + 1;
-        const int64_t base = D.cell(a, b, 0);
-        int32_t nc = 0;
-        int64_t rf = -1;
-        for (int64_t r = 0; r <= D.Pr(); ++r) {
-            const bool fl = r < D.Pr() && type[base + r] == 2;
-            if (fl && rf < 0) rf = r;
-            if (!fl && rf >= 0) {
-                const int64_t r0 = rf & ~int64_t(1), r1 = (r - 1) | 1;
-                nc += (int32_t)((r1 - r0 + 1 + piece - 1) / piece);
-                rf = -1;
-            }
+        const int a = (int)(c / D.Nb) + 1, b = (int)(c % D.Nb) + 1;
+        int left = (int)(i - F.off[c]), rf = -1, re = -1;
+        for_each_run(A, a, b, [&](int f, int e) {
+            const int n = run_pieces(f, e, F.piece, PAIR);
+            if (left < n) { rf = f; re = e; return false; }
+            left -= n;
+            return true;
+        });
+        if (rf < 0) { atomicOr(F.err, 1); continue; }
+        const int r0 = (PAIR ? rf & ~1 : rf) + left * F.piece, r1 = PAIR ? re | 1 : re;
+        const int len = min(F.piece, r1 - r0 + 1);
+        const int lf = max(r0, rf), ll = min(r0 + len - 1, re);    // fluid levels of the piece
+        Chunk ch;
+        const int32_t n0 = A.id(a, b, r0);
+        ch.n0 = (int32_t)(F.node_off + n0);
+        ch.len_inst = (uint32_t)len | ((uint32_t)F.inst << 8);
+        ch.vmask = ch.wmask = ch.zmask = ch.bmask = 0;
+        // the piece's own nodes and the levels next to its fluid ones have consecutive ids
+        if (n0 < 1 || A.id(a, b, r0 + len - 1) != n0 + len - 1 || A.id(a, b, lf - 1) != n0 + (lf - 1 - r0) ||
+            A.id(a, b, ll + 1) != n0 + (ll + 1 - r0) || (PAIR && ((n0 & 1) || (r0 & 1)))) {
+            atomicOr(F.err, 1);
+            continue;
         }
-        nchunk[c] = nc;
-    }
-}
-
-__global__ void k_col_fill2(FillArgs A) {
-    const Pad& D = A.D;
-    const int64_t ncol = (int64_t)D.Na * D.Nb;
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncol; c += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t a = c / D.Nb + 1, b = c % D.Nb + 1;
-        const int64_t base = D.cell(a, b, 0);
-        int64_t out = A.chunk_off[c];
-        int64_t ms = A.mslot_off[c];
-        int64_t rf = -1;
-        for (int64_t r = 0; r <= D.Pr(); ++r) {
-            const bool fl = r < D.Pr() && A.type[base + r] == 2;
-            if (fl && rf < 0) rf = r;
-            if (fl || rf < 0) continue;
-            const int64_t re = r - 1;
-            const int64_t r1 = re | 1;
-            for (int64_t r0 = rf & ~int64_t(1); r0 <= r1; r0 += A.piece) {
-                const int len = (int)std::min<int64_t>(A.piece, r1 - r0 + 1);
-                const int64_t lf = std::max(r0, rf), ll = std::min(r0 + len - 1, re);   // fluid levels of the piece
-                Chunk ch;
-                const int32_t n0 = A.node_of_cell[base + r0];
-                ch.n0 = (int32_t)(A.node_off + n0);
-                ch.len_inst = (uint32_t)len | ((uint32_t)A.inst << 8);
-                ch.vmask = ch.wmask = ch.zmask = ch.bmask = 0;
-                ch.mslot0 = (int32_t)(A.mslot_base + ms);
-                if ((n0 & 1) || (r0 & 1) || A.node_of_cell[base + r0 + len - 1] != n0 + len - 1 ||
-                    A.node_of_cell[base + lf - 1] != n0 + (int32_t)(lf - 1 - r0) ||
-                    A.node_of_cell[base + ll + 1] != n0 + (int32_t)(ll + 1 - r0))
-                    atomicOr(A.err, 1);
-                for (int64_t lv = lf; lv <= ll; ++lv) {
-                    const int j = (int)(lv - r0);
-                    ch.vmask |= 1u << j;
-                    const int ro = A.role[n0 + j];
-                    if (ro == 1) ch.wmask |= 1u << j;
-                    if (ro >= 1) { ch.bmask |= 1u << j; ++ms; }
-                }
-                const int64_t zfirst = lower_bound_i64(A.znodes, A.nz, n0);
-                ch.zslot0 = (int32_t)(A.zslot_off + zfirst);
-                for (int64_t zz = zfirst; zz < A.nz && A.znodes[zz] < n0 + len; ++zz)
-                    ch.zmask |= 1u << (int)(A.znodes[zz] - n0);
-                for (int da = -1; da <= 1; ++da)
-                    for (int db = -1; db <= 1; ++db) {
-                        if (da == 0 && db == 0) continue;
-                        // virtual id of level r0-1 such that K + 1 + (level - r0) is the id of
-                        // every level of the fluid window lf-1 .. ll+1 (checked at both ends)
-                        const int32_t kf = A.node_of_cell[D.cell(a + da, b + db, lf - 1)];
-                        const int32_t kl = A.node_of_cell[D.cell(a + da, b + db, ll + 1)];
-                        const int32_t k = kf - (int32_t)(lf - r0);
-                        // (k + 1 is the id of level r0: even, like every id of an even level)
-                        if (kf < 0 || kl != k + 1 + (int32_t)(ll + 1 - r0) || ((k + 1) & 1)) atomicOr(A.err, 1);
-                        ch.K[col8(da, db)] = (int32_t)(A.node_off + (kf < 0 ? 0 : k));
-                    }
-                A.chunks[out++] = ch;
-            }
-            rf = -1;
+        ch.mslot0 = (int32_t)(F.mslot_base + F.brank[n0 + (lf - r0)]);
+        for (int lv = lf; lv <= ll; ++lv) {
+            const int j = lv - r0;
+            ch.vmask |= 1u << j;
+            const int ro = F.role[n0 + j];
+            if (ro == 1) ch.wmask |= 1u << j;
+            if (ro >= 1) ch.bmask |= 1u << j;
         }
+        const int64_t zfirst = lower_bound_i64(F.znodes, F.nz, n0);
+        ch.zslot0 = (int32_t)(F.zslot_off + zfirst);
+        for (int64_t zz = zfirst; zz < F.nz && F.znodes[zz] < n0 + len; ++zz) ch.zmask |= 1u << (int)(F.znodes[zz] - n0);
+        for (int da = -1; da <= 1; ++da)
+            for (int db = -1; db <= 1; ++db) {
+                if (da == 0 && db == 0) continue;
+                // virtual id of level r0-1 such that K + 1 + (level - r0) is the id of
+                // every level of the fluid window lf-1 .. ll+1 (checked at both ends)
+                const int32_t kf = A.id(a + da, b + db, lf - 1), kl = A.id(a + da, b + db, ll + 1);
+                const int32_t k = kf - (lf - r0);
+                // (paired: k + 1 is the id of level r0, even, like every id of an even level)
+                if (kf < 0 || kl != k + 1 + (ll + 1 - r0) || (PAIR && ((k + 1) & 1))) atomicOr(F.err, 1);
+                ch.K[col8(da, db)] = (int32_t)(F.node_off + (kf < 0 ? 0 : k));
+            }
+        F.chunks[i] = ch;
     }
 }
 
@@ -690,32 +645,31 @@ Vel make_vel(int Q, int ra) {
     return v;
 }
 
-// Chunk count of a run axis straight from the x-major fluid flags (no
-// permutation, no node typing): the fluid runs along the axis, each cut into
-// pieces of `piece` slots, widened to whole pairs of padded levels when
-// `pairs` (the paired kernel's pieces, k_col_count2); summed into *total.
-__global__ void k_count_runs(const uint8_t* __restrict__ flags, int Nx, int Ny, int Nz, int ra, int piece, int pairs,
-                             unsigned long long* __restrict__ total) {
-    const int64_t nb = ra == 2 ? Ny : Nz, len = ra == 2 ? Nz : Ny, stride = ra == 2 ? 1 : Nz;
-    const int64_t ncol = (int64_t)Nx * nb;
+// Pieces of a run axis straight from its fluid bits, summed into *total.
+__global__ void k_count_runs(Lattice A, int piece, int pairs, unsigned long long* __restrict__ total) {
+    const int64_t ncol = (int64_t)A.D.Na * A.D.Nb;
     unsigned long long cnt = 0;
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncol; c += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t x = c / nb, b = c % nb;
-        const int64_t base = ra == 2 ? (x * Ny + b) * Nz : x * (int64_t)Ny * Nz + b;
-        int64_t rf = -1;
-        for (int64_t r = 0; r <= len; ++r) {
-            const bool fl = r < len && flags[base + r * stride] != 0;
-            if (fl && rf < 0) rf = r;
-            if (!fl && rf >= 0) {
-                int64_t lo = rf + 1, hi = r;                 // padded levels of the run
-                if (pairs) { lo &= ~int64_t(1); hi |= 1; }
-                cnt += (unsigned long long)((hi - lo + piece) / piece);
-                rf = -1;
-            }
-        }
-    }
+    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncol; c += (int64_t)gridDim.x * blockDim.x)
+        for_each_run(A, (int)(c / A.D.Nb) + 1, (int)(c % A.D.Nb) + 1, [&](int rf, int re) {
+            cnt += (unsigned long long)run_pieces(rf, re, piece, pairs != 0);
+            return true;
+        });
     for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
     if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(total, cnt);
+}
+
+// The fluid bits along the run axis: the geometry's own words for z, transposed
+// into `own` for y.
+lbm_status run_axis_bits(const lbm_geometry* g, const Perm& P, DBuf<uint32_t>& own, const uint32_t** out, cudaStream_t st) {
+    const uint32_t* z = geometry_fluid_dev(g);
+    *out = z;
+    if (P.ra == 2) return LBM_OK;
+    LBM_TRY(own.alloc((int64_t)P.Nx * P.Nz * words_for(P.Ny), "fluid bits", st));
+    const int64_t warps = (int64_t)P.Nx * words_for(P.Ny) * words_for(P.Nz);
+    k_transpose_bits<<<blocks_for(warps * 32, 256), 256, 0, st>>>(z, P.Nx, P.Ny, P.Nz, own.p);
+    LBM_CUDA(cudaGetLastError());
+    *out = own.p;
+    return LBM_OK;
 }
 
 // Number of chunks of the step kernel in use (paired pieces of `piece`
@@ -723,12 +677,15 @@ __global__ void k_count_runs(const uint8_t* __restrict__ flags, int Nx, int Ny, 
 lbm_status count_chunks(const lbm_geometry* g, int ra, int piece, bool pairs, cudaStream_t st, int64_t* n) {
     int dims[3];
     geometry_dims(g, dims);
+    const Perm P{ra, dims[0], dims[1], dims[2]};
     DBuf<unsigned long long> tot;
+    DBuf<uint32_t> bits;
+    Lattice A{};
+    A.D = Pad{P.Na(), P.Nb(), P.Nr()};
+    LBM_TRY(run_axis_bits(g, P, bits, &A.fluid, st));
     LBM_TRY(tot.alloc(1, "chunk count", st));
     LBM_CUDA(cudaMemsetAsync(tot.p, 0, sizeof(unsigned long long), st));
-    const int64_t ncol = (int64_t)dims[0] * (ra == 2 ? dims[1] : dims[2]);
-    k_count_runs<<<blocks_for(ncol, 128), 128, 0, st>>>(geometry_flags_dev(g), dims[0], dims[1], dims[2], ra, piece,
-                                                          pairs ? 1 : 0, tot.p);
+    k_count_runs<<<blocks_for((int64_t)P.Na() * P.Nb(), 128), 128, 0, st>>>(A, piece, pairs ? 1 : 0, tot.p);
     LBM_CUDA(cudaGetLastError());
     unsigned long long h = 0;
     LBM_CUDA(cudaMemcpyAsync(&h, tot.p, sizeof h, cudaMemcpyDeviceToHost, st));
@@ -743,48 +700,36 @@ lbm_status build_instance(const lbm_geometry* g, const lbm_sim_params* p, int Q,
     int dims[3];
     geometry_dims(g, dims);
     const Perm P{ra, dims[0], dims[1], dims[2]};
-    const int64_t npts = (int64_t)dims[0] * dims[1] * dims[2];
-    const uint8_t* flags = geometry_flags_dev(g);
-    DBuf<uint8_t> fperm;
-    const uint8_t* pflags = flags;
-    if (ra != 2) {
-        LBM_TRY(fperm.alloc(npts, "permuted flags", st));
-        k_permute_flags<<<blocks_for(npts, 256), 256, 0, st>>>(flags, P, fperm.p);
-        pflags = fperm.p;
-    }
-    // 1. fluid + ghost nodes on the padded grid, numbered in permuted order
-    const Pad D{P.Na(), P.Nb(), P.Nr()};
-    DBuf<uint8_t> type;
-    LBM_TRY(type.alloc(D.cells(), "node types", st));
-    LBM_TRY(compute_types(pflags, D, type.p, st));
-    k_parity_ghosts<<<blocks_for(D.cells(), 256), 256, 0, st>>>(D, type.p);
-    int64_t* nc = nullptr;
-    LBM_TRY(scan::compact(type.p, D.cells(), &nc, &out.N, st));
-    DBuf<int64_t> node_cell; node_cell.adopt(nc, st);
+    // 1. fluid + ghost nodes on the padded grid, numbered in column order
+    DBuf<uint32_t> ubits, nbits, nrank, zrank;
+    Lattice A{};
+    A.D = Pad{P.Na(), P.Nb(), P.Nr()};
+    LBM_TRY(run_axis_bits(g, P, ubits, &A.fluid, st));
+    const int64_t nw = A.D.words();
+    LBM_TRY(nbits.alloc(nw, "node bits", st));
+    LBM_TRY(nrank.alloc(nw, "node ranks", st));
+    k_node_bits<<<blocks_for(nw, 256), 256, 0, st>>>(A, nbits.p);
+    LBM_TRY(scan::bit_ranks(nbits.p, nw, nrank.p, &out.N, st));
     if (node_off + out.N >= INT32_MAX) return fail(LBM_ERR_ARG, "more than 2^31 lattice nodes");
-    DBuf<int32_t> noc;
-    LBM_TRY(noc.alloc(D.cells(), "node map", st));
-    LBM_CUDA(cudaMemsetAsync(noc.p, 0xff, sizeof(int32_t) * D.cells(), st));
-    k_scatter_ids<<<blocks_for(out.N, 256), 256, 0, st>>>(nc, out.N, noc.p);
-    // 2. outputs in x-major order (the reference's node order, Subdomain.cpp:638-651)
-    {
-        int64_t* xg = nullptr;
-        LBM_TRY(scan::compact(flags, npts, &xg, &out.NF, st));
-        out.node_grid.adopt(xg, st);
-        if (out.NF == 0) return fail(LBM_ERR_ARG, "instance %d has no fluid node", inst);
-        DBuf<int32_t> rank;
-        LBM_TRY(rank.alloc(npts, "rank map", st));
-        k_scatter_ids<<<blocks_for(out.NF, 256), 256, 0, st>>>(xg, out.NF, rank.p);
-        LBM_TRY(out.out_pos.alloc(out.N, "output positions", st));
-        k_out_pos<<<blocks_for(out.N, 256), 256, 0, st>>>(nc, out.N, type.p, D, P, rank.p, out_off, out.out_pos.p);
-    }
-    // 3. roles
+    A.nodes = nbits.p;
+    A.rank = nrank.p;
+    // 2. outputs in x-major order (the reference's node order, Subdomain.cpp:638-651) and roles
+    const uint32_t* zfluid = geometry_fluid_dev(g);
+    const int Wz = words_for(dims[2]);
+    const int64_t zw = (int64_t)dims[0] * dims[1] * Wz;
+    LBM_TRY(zrank.alloc(zw, "output ranks", st));
+    LBM_TRY(scan::bit_ranks(zfluid, zw, zrank.p, &out.NF, st));
+    if (out.NF == 0) return fail(LBM_ERR_ARG, "instance %d has no fluid node", inst);
+    LBM_TRY(out.node_grid.alloc(out.NF, "node grid indices", st));
+    k_points<<<blocks_for(zw, 256), 256, 0, st>>>(zfluid, zrank.p, zw, Wz, dims[2], out.node_grid.p);
     DBuf<int8_t> role;
     LBM_TRY(role.alloc(out.N, "node roles", st));
-    k_roles_fluid<<<blocks_for(out.N, 256), 256, 0, st>>>(nc, out.N, type.p, role.p);
+    LBM_TRY(out.out_pos.alloc(out.N, "output positions", st));
+    k_nodes<<<blocks_for(nw, 256), 256, 0, st>>>(A, P, zfluid, zrank.p, out_off, role.p, out.out_pos.p);
+    // 3. boundary roles
     const int64_t nb = geometry_nboundary(g);
     if (nb)
-        k_roles<<<blocks_for(nb, 256), 256, 0, st>>>(geometry_bidx_dev(g), geometry_bmask_dev(g), nb, P, D, noc.p, role.p);
+        k_roles<<<blocks_for(nb, 256), 256, 0, st>>>(geometry_bidx_dev(g), geometry_bmask_dev(g), nb, A, P, role.p);
     // 4. Zou-He nodes: role list with a boundary-condition kind
     int kind[64] = {0};
     const lbm_list_bc* lbc[64] = {nullptr};
@@ -850,45 +795,44 @@ lbm_status build_instance(const lbm_geometry* g, const lbm_sim_params* p, int Q,
                             (long long)rank[l]);
         }
     }
-    // 5. chunks and missing masks
-    const int64_t ncol = (int64_t)D.Na * D.Nb;
-    DBuf<int32_t> ccount, bcount;
-    DBuf<int64_t> coff, moff;
-    LBM_TRY(ccount.alloc(ncol, "chunk counts", st));
-    LBM_TRY(bcount.alloc(ncol, "boundary counts", st));
-    LBM_TRY(coff.alloc(ncol, "chunk offsets", st));
-    LBM_TRY(moff.alloc(ncol, "mask offsets", st));
-    k_col_count<<<blocks_for(ncol, 128), 128, 0, st>>>(type.p, noc.p, role.p, D, ccount.p, bcount.p);
-    LBM_TRY(scan::exclusive_scan(ccount.p, ncol, coff.p, &out.nchunks, st));
-    LBM_TRY(scan::exclusive_scan(bcount.p, ncol, moff.p, &out.nmask, st));
-    LBM_TRY(out.chunks.alloc(out.nchunks, "chunks", st));
+    // 5. missing masks and pieces: chunks of 32 nodes, and paired pieces of every
+    // size (the autotuner may switch sizes; they share the masks, same node order)
+    const int64_t ncol = (int64_t)A.D.Na * A.D.Nb;
+    DBuf<uint8_t> bflag;
+    DBuf<uint32_t> brank;
+    LBM_TRY(bflag.alloc(out.N, "boundary flags", st));
+    LBM_TRY(brank.alloc(out.N, "boundary ranks", st));
+    k_boundary_flag<<<blocks_for(out.N, 256), 256, 0, st>>>(role.p, out.N, bflag.p);
+    LBM_TRY(scan::exclusive_scan(bflag.p, out.N, brank.p, &out.nmask, st));
     LBM_TRY(out.mmask.alloc(out.nmask, "missing masks", st));
+    k_masks<<<blocks_for(nw, 256), 256, 0, st>>>(A, make_vel(Q, ra), role.p, brank.p, out.mmask.p);
+    const int tables = npl == 2 ? 4 : 1;
+    DBuf<int32_t> counts[4];
+    PieceCounts pc{};
+    for (int k = 0; k < tables; ++k) {
+        LBM_TRY(counts[k].alloc(ncol, "piece counts", st));
+        pc.n[k] = counts[k].p;
+    }
+    k_piece_counts<<<blocks_for(ncol, 128), 128, 0, st>>>(A, tables, pc);
+    DBuf<int64_t> off[4];
     FillArgs fa;
-    fa.type = type.p; fa.node_of_cell = noc.p; fa.role = role.p; fa.D = D; fa.V = make_vel(Q, ra);
-    fa.chunk_off = coff.p; fa.mslot_off = moff.p;
+    fa.A = A; fa.role = role.p; fa.brank = brank.p;
     fa.znodes = zn; fa.nz = nzn; fa.node_off = node_off; fa.zslot_off = zslot_off; fa.mslot_base = mslot_off;
-    fa.inst = inst; fa.chunks = out.chunks.p; fa.mmask = out.mmask.p; fa.err = d_err;
-    k_col_fill<<<blocks_for(ncol, 128), 128, 0, st>>>(fa);
-    LBM_CUDA(cudaGetLastError());
-    if (npl == 2) {
-        // paired chunks of every piece size (the autotuner may switch sizes);
-        // they share the missing masks (same boundary-node order)
-        for (int k = 0; k < 3; ++k) {
-            const int pc = 8 << k;
-            DBuf<int64_t> coff2;
-            LBM_TRY(coff2.alloc(ncol, "paired chunk offsets", st));
-            k_col_count2<<<blocks_for(ncol, 128), 128, 0, st>>>(type.p, D, pc, ccount.p);
-            LBM_TRY(scan::exclusive_scan(ccount.p, ncol, coff2.p, &out.nchunks2[k], st));
-            LBM_TRY(out.chunks2[k].alloc(out.nchunks2[k], "paired chunks", st));
-            FillArgs f2 = fa;
-            f2.chunk_off = coff2.p;
-            f2.chunks = out.chunks2[k].p;
-            f2.mmask = nullptr;
-            f2.piece = pc;
-            k_col_fill2<<<blocks_for(ncol, 128), 128, 0, st>>>(f2);
-            LBM_CUDA(cudaGetLastError());
-            LBM_CUDA(cudaStreamSynchronize(st));   // coff2 is freed on return
-        }
+    fa.inst = inst; fa.err = d_err;
+    for (int k = 0; k < tables; ++k) {
+        DBuf<Chunk>& tab = k == 0 ? out.chunks : out.chunks2[k - 1];
+        int64_t& n = k == 0 ? out.nchunks : out.nchunks2[k - 1];
+        LBM_TRY(off[k].alloc(ncol, "piece offsets", st));
+        LBM_TRY(scan::exclusive_scan(counts[k].p, ncol, off[k].p, &n, st));
+        LBM_TRY(tab.alloc(n, "pieces", st));
+        fa.off = off[k].p;
+        fa.pieces = n;
+        fa.piece = k == 0 ? 32 : 4 << k;
+        fa.chunks = tab.p;
+        if (n == 0) continue;
+        if (k == 0) k_fill_pieces<false><<<blocks_for(n, 128), 128, 0, st>>>(fa);
+        else k_fill_pieces<true><<<blocks_for(n, 128), 128, 0, st>>>(fa);
+        LBM_CUDA(cudaGetLastError());
     }
     int32_t herr = 0;
     LBM_CUDA(cudaMemcpyAsync(&herr, d_err, sizeof herr, cudaMemcpyDeviceToHost, st));
