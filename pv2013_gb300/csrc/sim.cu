@@ -521,22 +521,61 @@ struct MonOut {
     int32_t bad;
 };
 
-__global__ void k_reduce_partials(Partials p, int64_t nblocks, MonOut* out) {
-    // fixed-order reduction: thread t sums a contiguous range, then a
-    // fixed tree over 256 threads (deterministic for a given block count)
-    __shared__ double s[4][256];
-    __shared__ int sb[256];
-    const int t = threadIdx.x;
-    const int64_t per = (nblocks + 255) / 256;
+// Fixed-order reduction of the block partials (deterministic for a given block
+// count): range t of 256 contiguous ranges in order, then a fixed tree over
+// the 256 sums.  One SM's FP64 rate bounds the ranges, so beyond 4096 blocks
+// they are summed on 32 SMs first (96 533 blocks: 255 us in one block, 119 us).
+constexpr int kReduceRanges = 256;
+struct RangeSum {
+    double a[4];
+    int32_t bad;
+};
+__device__ __forceinline__ RangeSum reduce_range(const Partials& p, int64_t nblocks, int t) {
+    const int64_t per = (nblocks + kReduceRanges - 1) / kReduceRanges;
     const int64_t b = t * per, e = min(nblocks, b + per);
-    double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-    int bb = 0;
-    for (int64_t i = b; i < e; ++i) {
-        a0 += p.mass[i]; a1 += p.inflow[i]; a2 += p.outflow[i]; a3 = fmax(a3, p.maxu[i]); bb |= p.bad[i];
+    RangeSum s = {{0.0, 0.0, 0.0, 0.0}, 0};
+    constexpr int U = 8;                             // loads in flight per array
+    for (int64_t i = b; i < e; i += U) {
+        double v[4][U];
+        int32_t bad[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const int64_t j = min(i + k, e - 1);
+            v[0][k] = p.mass[j]; v[1][k] = p.inflow[j]; v[2][k] = p.outflow[j]; v[3][k] = p.maxu[j]; bad[k] = p.bad[j];
+        }
+#pragma unroll
+        for (int k = 0; k < U; ++k)
+            if (i + k < e) {
+                s.a[0] += v[0][k]; s.a[1] += v[1][k]; s.a[2] += v[2][k]; s.a[3] = fmax(s.a[3], v[3][k]); s.bad |= bad[k];
+            }
     }
-    s[0][t] = a0; s[1][t] = a1; s[2][t] = a2; s[3][t] = a3; sb[t] = bb;
+    return s;
+}
+struct RangeOut {
+    double a[kReduceRanges][4];
+    int32_t bad[kReduceRanges];
+};
+__global__ void k_reduce_ranges(Partials p, int64_t nblocks, RangeOut* __restrict__ out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const RangeSum s = reduce_range(p, nblocks, t);
+    for (int k = 0; k < 4; ++k) out->a[t][k] = s.a[k];
+    out->bad[t] = s.bad;
+}
+__global__ void k_reduce_partials(Partials p, int64_t nblocks, const RangeOut* __restrict__ ranges, MonOut* out) {
+    __shared__ double s[4][kReduceRanges];
+    __shared__ int sb[kReduceRanges];
+    const int t = threadIdx.x;
+    RangeSum r;
+    if (ranges) {
+        for (int k = 0; k < 4; ++k) r.a[k] = ranges->a[t][k];
+        r.bad = ranges->bad[t];
+    } else {
+        r = reduce_range(p, nblocks, t);
+    }
+    for (int k = 0; k < 4; ++k) s[k][t] = r.a[k];
+    sb[t] = r.bad;
     __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
+    for (int o = kReduceRanges / 2; o > 0; o >>= 1) {
         if (t < o) {
             s[0][t] += s[0][t + o]; s[1][t] += s[1][t + o]; s[2][t] += s[2][t + o];
             s[3][t] = fmax(s[3][t], s[3][t + o]); sb[t] |= sb[t + o];
@@ -603,6 +642,7 @@ struct lbm_sim {
     // monitors
     double* part = nullptr;        // 4 * nblocks doubles
     int32_t* partbad = nullptr;
+    RangeOut* ranges = nullptr;    // sums of the partials' ranges
     MonOut* mon = nullptr;
     int64_t part_blocks = 0;
     double mass0 = 0.0;
@@ -950,7 +990,11 @@ lbm_status sim_dry(lbm_sim* S, double* of, double* orho, double* ou, bool partia
     if (S->pattern == LBM_PULL) { mode = MODE_PULL; src = S->buf[S->cur]; }
     else { mode = aa_mode(S); src = S->buf[0]; }
     LBM_TRY(sim_launch(S, mode, true, src, src, S->steps_done, nullptr, p, of, orho, ou, st));
-    if (partials) k_reduce_partials<<<1, 256, 0, st>>>(p, S->part_blocks, S->mon);
+    if (partials) {
+        const bool split = S->part_blocks > 4096;
+        if (split) k_reduce_ranges<<<32, kReduceRanges / 32, 0, st>>>(p, S->part_blocks, S->ranges);
+        k_reduce_partials<<<1, kReduceRanges, 0, st>>>(p, S->part_blocks, split ? S->ranges : nullptr, S->mon);
+    }
     LBM_CUDA(cudaGetLastError());
     return LBM_OK;
 }
@@ -1213,6 +1257,7 @@ lbm_status sim_create(const lbm_geometry* const* g, const lbm_sim_params* p, siz
     LBM_CUDA(cudaMalloc(&S->part, sizeof(double) * 4 * S->part_blocks));
     LBM_CUDA(cudaMalloc(&S->partbad, sizeof(int32_t) * S->part_blocks));
     LBM_CUDA(cudaMalloc(&S->mon, sizeof(MonOut)));
+    LBM_CUDA(cudaMalloc(&S->ranges, sizeof(RangeOut)));
     LBM_CUDA(cudaMalloc(&S->step_base, sizeof(int64_t)));
     LBM_CUDA(cudaGetLastError());
     LBM_CUDA(cudaStreamSynchronize(st));
@@ -2040,6 +2085,7 @@ void lbm_sim_destroy(lbm_sim* S) {
     if (S->part) cudaFree(S->part);
     if (S->partbad) cudaFree(S->partbad);
     if (S->mon) cudaFree(S->mon);
+    if (S->ranges) cudaFree(S->ranges);
     if (S->step_base) cudaFree(S->step_base);
     if (S->err) cudaFree(S->err);
     delete S;

@@ -310,27 +310,6 @@ __host__ __device__ constexpr bool is_velocity_kind(int kind) {
     return kind == LBM_BC_VEL_NEGY || kind == LBM_BC_VEL_POSX || kind == LBM_BC_VELOCITY;
 }
 
-// rho and u from plain populations with the reference's grouped sums
-// (Simulation.cpp:32-79 for D3Q19, :82-148 for D3Q27).
-template <int Q, class T>
-__device__ __forceinline__ void macro_ref(const T* f, T& rho, T& ux, T& uy, T& uz) {
-    rho = T(0.0);
-#pragma unroll
-    for (int q = 0; q < Q; ++q) rho += f[q];
-    if constexpr (Q == 19) {
-        ux = ((f[0] + f[6] + f[7] + f[8] + f[9]) - (f[1] + f[10] + f[11] + f[12] + f[13])) / rho;
-        uy = ((f[2] + f[6] + f[10] + f[14] + f[15]) - (f[3] + f[7] + f[11] + f[16] + f[17])) / rho;
-        uz = ((f[4] + f[8] + f[12] + f[14] + f[16]) - (f[5] + f[9] + f[13] + f[15] + f[17])) / rho;
-    } else {
-        ux = ((f[1] + f[7] + f[8] + f[11] + f[13] + f[19] + f[21] + f[23] + f[25]) -
-              (f[2] + f[9] + f[10] + f[12] + f[14] + f[20] + f[22] + f[24] + f[26])) / rho;
-        uy = ((f[3] + f[7] + f[9] + f[15] + f[16] + f[19] + f[21] + f[24] + f[26]) -
-              (f[4] + f[8] + f[10] + f[17] + f[18] + f[20] + f[22] + f[23] + f[25])) / rho;
-        uz = ((f[5] + f[11] + f[12] + f[15] + f[17] + f[19] + f[22] + f[23] + f[26]) -
-              (f[6] + f[13] + f[14] + f[16] + f[18] + f[20] + f[21] + f[24] + f[25])) / rho;
-    }
-}
-
 // ---------------------------------------------------------------------------
 // FP64: the reference's results with fewer operations.  GB300 retires about 2
 // FP64 operations per clock and SM, which bounds every FP64 kernel here, so the
@@ -384,6 +363,40 @@ __device__ __forceinline__ void moments_ref(const T* f, T& rho, T& jx, T& jy, T&
         jz = (f[5] + f[11] + f[12] + f[15] + f[17] + f[19] + f[22] + f[23] + f[26]) -
              (f[6] + f[13] + f[14] + f[16] + f[18] + f[20] + f[21] + f[24] + f[25]);
     }
+}
+
+// rho and u of a node in FP64, from its populations as stored (Simulation.cpp:32-79,
+// :82-148): snapshots and monitors, bound by their FP64 operations (see above).
+// A stored FP32 population is widened by moving its bits: shifted into place
+// they are the value times 2^-896, a normal number or an exact subnormal, so every
+// sum rounds as it would unscaled; four products scale the sums back.  (A
+// conversion each is 19 or 27 FP64-rate instructions.)  A population that is
+// infinite or NaN takes the conversions.  With this, one reciprocal, and the speed's
+// root once per block, the monitor launch of the vascular tree takes 2.0 ms
+// (3.75), the D3Q27 snapshot of the bifurcation 255 us (437).
+template <int Q, int S>
+__device__ __forceinline__ void macro_out(const typename Work<S>::T* f, double& rho, double& ux, double& uy, double& uz) {
+    double p[Q], jx, jy, jz;
+    if constexpr (S == ST_F64) {
+        moments_ref<Q, double>(f, rho, jx, jy, jz);
+    } else {
+        uint32_t top = 0;                            // bit 31: an exponent of all ones
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const uint32_t b = __float_as_uint(plain<S, Q>(f[q], q));
+            top |= (b & 0x7f800000u) + 0x00800000u;
+            p[q] = __hiloint2double((int)((b & 0x80000000u) | ((b >> 3) & 0x0fffffffu)), (int)(b << 29));
+        }
+        double scale = 0x1p896;
+        if (top & 0x80000000u) {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) p[q] = (double)plain<S, Q>(f[q], q);
+            scale = 1.0;
+        }
+        moments_ref<Q, double>(p, rho, jx, jy, jz);
+        rho *= scale; jx *= scale; jy *= scale; jz *= scale;
+    }
+    div3(jx, jy, jz, rho, ux, uy, uz);
 }
 
 // FP64 BGK collision, the reference's rounding on every population
@@ -501,7 +514,7 @@ __device__ __forceinline__ uint32_t lane_missing(const StepArgs& a, const Chunk*
 template <int Q, int S, int MODE, bool DRY>
 __device__ __forceinline__ void node_update(const StepArgs& a, int32_t zslot0, typename Work<S>::T* f, uint32_t missing,
                                             uint32_t wmask, uint32_t zmask, int lane, int32_t n, int inst, int64_t step,
-                                            double* mon) {
+                                            double* mon, bool want_mon) {
     using L = Lat<Q>;
     using T = typename Work<S>::T;
     const void* A = a.src;
@@ -551,35 +564,32 @@ __device__ __forceinline__ void node_update(const StepArgs& a, int32_t zslot0, t
         for (int q = 0; q < Q; ++q) f[q] = unplain<S, Q>(p[q], q);
     }
     if constexpr (DRY) {
-        double fp[Q];
-#pragma unroll
-        for (int q = 0; q < Q; ++q) fp[q] = (double)plain<S, Q>(f[q], q);
         double rho, ux, uy, uz;
-        macro_ref<Q, double>(fp, rho, ux, uy, uz);
+        macro_out<Q, S>(f, rho, ux, uy, uz);
         const int64_t pos = (int64_t)a.out_pos[n];
         if (a.out_f) {
 #pragma unroll
-            for (int q = 0; q < Q; ++q) a.out_f[pos * Q + q] = fp[q];
+            for (int q = 0; q < Q; ++q) a.out_f[pos * Q + q] = (double)plain<S, Q>(f[q], q);
         }
         if (a.out_rho) a.out_rho[pos] = rho;
         if (a.out_u) { a.out_u[3 * pos] = ux; a.out_u[3 * pos + 1] = uy; a.out_u[3 * pos + 2] = uz; }
-        const double sp = sqrt(ux * ux + uy * uy + uz * uz);
-        mon[0] = rho;
-        mon[3] = sp;
-        mon[4] = (isfinite(rho) && isfinite(sp)) ? 0.0 : 1.0;
-        if (zl) {
-            if (zdir > 0) mon[1] = rho * sp;
-            else mon[2] = rho * sp;
+        if (want_mon) {
+            const double sp2 = ux * ux + uy * uy + uz * uz;
+            mon[0] = rho;
+            mon[3] = sp2;
+            mon[4] = (isfinite(rho) && isfinite(sp2)) ? 0.0 : 1.0;
+            if (zl) mon[zdir > 0 ? 1 : 2] = rho * sqrt(sp2);
         }
     } else {
         collide<Q, S>(f, a.insts[inst]);
     }
 }
 
-// FP64 holds two registers a population and is bound by its arithmetic: 128
-// registers without spills (64 spilled 40 to 1060 bytes) and 16 warps an SM
+// FP64 storage and the FP64 moments of the dry launches hold two registers a
+// population and are bound by their arithmetic: 128 registers without spills (64
+// spilled 40 to 1060 bytes) and 16 warps an SM
 template <int Q, int S, int MODE, bool DRY, int RA>
-__global__ void __launch_bounds__(256, S == ST_F64 ? 2 : 4) k_step(StepArgs a, Partials part) {
+__global__ void __launch_bounds__(256, S == ST_F64 || DRY ? 2 : 4) k_step(StepArgs a, Partials part) {
     using L = Lat<Q>;
     using X = Ax<Q, RA>;
     using T = typename Work<S>::T;
@@ -617,7 +627,7 @@ __global__ void __launch_bounds__(256, S == ST_F64 ? 2 : 4) k_step(StepArgs a, P
                 }
             }
             node_update<Q, S, MODE, DRY>(a, zmask ? __ldg(&cp->zslot0) : 0, f, missing, wmask, zmask, lane, n,
-                                         (int)(li >> 8), step, mon);
+                                         (int)(li >> 8), step, mon, DRY && part.mass != nullptr);
             if constexpr (!DRY) {
                 void* D = a.dst;
 #pragma unroll
@@ -644,28 +654,37 @@ __global__ void __launch_bounds__(256, S == ST_F64 ? 2 : 4) k_step(StepArgs a, P
     }
     if constexpr (DRY) {
         if (part.mass) {
-            // deterministic block reduction: warp shuffles then thread 0
+            // deterministic block reduction: warp shuffles then thread 0.  The
+            // fluxes are summed only in warps with an inlet or outlet node;
+            // the largest speed is taken squared, as an integer (the order of
+            // non-negative numbers; NaN does not count), one root per block
             __shared__ double sm[4][8];
             __shared__ int sb[8];
-            double m_mass = mon[0], m_in = mon[1], m_out = mon[2], m_maxu = mon[3];
-            int m_bad = mon[4] != 0.0;
+            double m_mass = mon[0], m_in = mon[1], m_out = mon[2];
+            unsigned long long m_maxu = mon[3] == mon[3] ? (unsigned long long)__double_as_longlong(mon[3]) : 0ull;
+            const bool flux = __any_sync(0xffffffffu, mon[1] != 0.0 || mon[2] != 0.0);   // (NaN != 0)
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 m_mass += __shfl_down_sync(0xffffffffu, m_mass, o);
-                m_in += __shfl_down_sync(0xffffffffu, m_in, o);
-                m_out += __shfl_down_sync(0xffffffffu, m_out, o);
-                m_maxu = fmax(m_maxu, __shfl_down_sync(0xffffffffu, m_maxu, o));
-                m_bad |= __shfl_down_sync(0xffffffffu, m_bad, o);
+                if (flux) {
+                    m_in += __shfl_down_sync(0xffffffffu, m_in, o);
+                    m_out += __shfl_down_sync(0xffffffffu, m_out, o);
+                }
+                m_maxu = max(m_maxu, __shfl_down_sync(0xffffffffu, m_maxu, o));
             }
+            const int m_bad = __any_sync(0xffffffffu, mon[4] != 0.0);
             const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-            if (lane == 0) { sm[0][w] = m_mass; sm[1][w] = m_in; sm[2][w] = m_out; sm[3][w] = m_maxu; sb[w] = m_bad; }
+            if (lane == 0) {
+                sm[0][w] = m_mass; sm[1][w] = m_in; sm[2][w] = m_out; sb[w] = m_bad;
+                sm[3][w] = __longlong_as_double((long long)m_maxu);
+            }
             __syncthreads();
             if (threadIdx.x == 0) {
                 double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
                 int b = 0;
                 for (int i = 0; i < nw; ++i) { s0 += sm[0][i]; s1 += sm[1][i]; s2 += sm[2][i]; s3 = fmax(s3, sm[3][i]); b |= sb[i]; }
                 part.mass[blockIdx.x] = s0; part.inflow[blockIdx.x] = s1; part.outflow[blockIdx.x] = s2;
-                part.maxu[blockIdx.x] = s3; part.bad[blockIdx.x] = b;
+                part.maxu[blockIdx.x] = sqrt(s3); part.bad[blockIdx.x] = b;
             }
         }
     }

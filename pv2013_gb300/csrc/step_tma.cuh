@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(256) k_step_tma(StepArgs a, int32_t* err) {
                 f[q] = v;
             }
             double mon[5];
-            node_update<Q, S, MODE, false>(a, cp->zslot0, f, missing, wmask, zmask, lane, n, (int)(li >> 8), step, mon);
+            node_update<Q, S, MODE, false>(a, cp->zslot0, f, missing, wmask, zmask, lane, n, (int)(li >> 8), step, mon, false);
             void* D = a.dst;
             if constexpr (MODE == MODE_AA_ODD) {
                 // re-read the bases rather than hold them across the update
