@@ -293,11 +293,21 @@ template <int Q, int S, int MODE> struct PairMaxReg {
     static constexpr int value = (Q == 19 && S != ST_F32) ? (MODE == MODE_AA_ODD ? 72 : 64) : 128;
 };
 
-template <int Q, int S, int MODE, int RA>
+// CHAIN: programmatic dependent launch, for a lattice of at most one wave of
+// blocks stepped launch by launch.  The next step's blocks become resident while
+// this step runs, read the tables, which no launch writes, and wait for its end
+// before they touch populations or the step counter: the launch gap and the table
+// loads leave the step's critical path (186 056-node vessel, BF16: 10.3 -> 8.6 us
+// a step; 10 240-node pipe 7.2 -> 5.7 us).  Graph replay has shorter gaps (the
+// vessel 7.9 us without, 8.5 with), and on larger lattices the wait costs
+// registers and scheduling freedom (vascular tree: 191 -> 205 us), so those
+// launches take the kernel without it.
+template <int Q, int S, int MODE, int RA, bool CHAIN>
 __global__ void __launch_bounds__(256) __maxnreg__((PairMaxReg<Q, S, MODE>::value)) k_step2(StepArgs a) {
     using L = Lat<Q>;
     using X = Ax<Q, RA>;
     using W = typename PairWord<S>::W;
+    if constexpr (CHAIN) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31;
     // a chunk piece is served by 2^lg lanes (4, 8 or 16): 32 >> lg pieces per warp
     const int lg = a.piece_lg;
@@ -346,7 +356,8 @@ __global__ void __launch_bounds__(256) __maxnreg__((PairMaxReg<Q, S, MODE>::valu
     const uint32_t e = (uint32_t)(n0 + 2 * t);     // id of the lo node (even)
     const uint32_t st = (uint32_t)a.stride;
     const uint32_t sw = st >> 1, ew = (uint32_t)(n0 >> 1) + (uint32_t)t;   // word offsets: plane stride, the pair's word
-    const int64_t step = a.step + (a.step_base ? *a.step_base : 0);
+    int64_t step = 0;
+    if constexpr (!CHAIN) step = a.step + (a.step_base ? *a.step_base : 0);
     const void* A = a.src;
 
     // column bases (virtual id of level r0-1) of the eight neighbour columns
@@ -376,6 +387,10 @@ __global__ void __launch_bounds__(256) __maxnreg__((PairMaxReg<Q, S, MODE>::valu
     extern __shared__ __align__(16) unsigned char zsm[];
     W* buf = (W*)zsm + (threadIdx.x >> 5) * (Q * 32) + lane;
     int32_t* ksm = reinterpret_cast<int32_t*>((W*)zsm + (blockDim.x >> 5) * (Q * 32)) + (threadIdx.x >> 5) * 64;
+    if constexpr (CHAIN) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        step = a.step + (a.step_base ? *a.step_base : 0);
+    }
     if (act) {
         int32_t K[8];
         if constexpr (MODE != MODE_AA_EVEN) load_K(K, false);
@@ -596,8 +611,10 @@ static lbm_status launch_pair_one(const StepArgs& a, int wpb, cudaStream_t st) {
         return fail(LBM_ERR_CUDA, "paired step kernel: device %d not supported", dev);
     const size_t smem = (size_t)wpb * (Q * 32 * sizeof(typename PairWord<S>::W) + (MODE == MODE_AA_ODD ? 256 : 0));
     if (smem > 48 * 1024 && opted[dev] < (int)smem) {
-        const cudaError_t e = cudaFuncSetAttribute(k_step2<Q, S, MODE, RA>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(k_step2<Q, S, MODE, RA, false>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_step2<Q, S, MODE, RA, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "paired step kernel shared memory: %s", cudaGetErrorString(e));
         opted[dev] = (int)smem;
     }
@@ -607,7 +624,7 @@ static lbm_status launch_pair_one(const StepArgs& a, int wpb, cudaStream_t st) {
     if (resident[dev][wpb] == 0) {
         int sms = 0, nb = 0;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_step2<Q, S, MODE, RA>, 32 * wpb, smem) != cudaSuccess)
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_step2<Q, S, MODE, RA, false>, 32 * wpb, smem) != cudaSuccess)
             return fail(LBM_ERR_CUDA, "paired step kernel occupancy: %s", cudaGetErrorString(cudaGetLastError()));
         resident[dev][wpb] = sms * (nb > 0 ? nb : 1);
     }
@@ -619,7 +636,23 @@ static lbm_status launch_pair_one(const StepArgs& a, int wpb, cudaStream_t st) {
     // waves measured the same within 0.3 %)
     StepArgs b = a;
     b.pf_ahead = (int64_t)resident[dev][wpb] * per_block / (MODE == MODE_AA_ODD ? 1 : 2);
-    k_step2<Q, S, MODE, RA><<<(unsigned)(blocks > 0 ? blocks : 1), 32 * wpb, smem, st>>>(b);
+    const unsigned grid = (unsigned)(blocks > 0 ? blocks : 1);
+    if (a.step_base || blocks > resident[dev][wpb]) {
+        k_step2<Q, S, MODE, RA, false><<<grid, 32 * wpb, smem, st>>>(b);
+        return LBM_OK;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(32 * wpb);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_step2<Q, S, MODE, RA, true>, b);
+    if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "paired step launch: %s", cudaGetErrorString(e));
     return LBM_OK;
 }
 
