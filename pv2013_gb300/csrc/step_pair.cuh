@@ -285,12 +285,20 @@ __device__ __forceinline__ void collide2(const typename PairWord<S>::W* raw, flo
     }
 }
 
-// register budget per thread: D3Q19 with 16-bit storage holds one 32-bit
-// word per population; 64 registers for the node-local and pull patterns, 72
-// for the AA odd pattern (its scatter needs a few more; 72 keeps 28 warps per
-// SM); FP32 storage (two registers per word) and D3Q27 get 128.
+// Register budget per thread.  The launches wait on loads, so warps in flight
+// count until the spills of a tighter budget cost more.  D3Q19 with 16-bit storage
+// holds one 32-bit word per population: 64 registers for the node-local and pull
+// patterns, 72 for the AA odd pattern (its scatter needs a few more; 72 keeps
+// 28 warps per SM).  FP32 storage (two registers per word) and D3Q27 ran with 128;
+// us per step on a 983 733-node bifurcation / a 3.7 M-node ensemble, 128 -> chosen:
+//   D3Q19 FP32    pull 41.3 -> 40.1 / 165 -> 159, AA 28.7 -> 25.8 / 136 -> 127
+//                 with 80 (AA odd 72: 28.3 / 144; pull 72: 41.3 / 165)
+//   D3Q27 16-bit  pull 55.3 -> 47.8 / 264 -> 217 with 80; AA 33.1 -> 32.0 / 180 -> 172
+//                 with 80 even, 96 odd (96 / 80: 34.7 / 176, 112 / 88: 33.9 / 184)
+//   D3Q27 FP32    AA 52.2 -> 50.3 / 243 -> 227 with 96 (80 and 88 spill: 56.7 / 252)
 template <int Q, int S, int MODE> struct PairMaxReg {
-    static constexpr int value = (Q == 19 && S != ST_F32) ? (MODE == MODE_AA_ODD ? 72 : 64) : 128;
+    static constexpr int value = Q == 19 ? (S == ST_F32 ? 80 : (MODE == MODE_AA_ODD ? 72 : 64))
+                                         : (S == ST_F32 || MODE == MODE_AA_ODD ? 96 : 80);
 };
 
 // CHAIN: programmatic dependent launch, for a lattice of at most one wave of
