@@ -150,25 +150,28 @@ __device__ __forceinline__ int enum_box(const VoxGrid& g, double inv_s, const do
         r.j1 = (int)floor(fmax(fmin(fmax(wy[0], fmax(wy[1], wy[2])) + md, (double)(g.Ny - 1)), -1.0));
     }
     const bool empty = r.i0 > r.i1 || r.j0 > r.j1;
-    // vertices relative to the box's first column, FP32: small numbers, error below 1e-6 of the extent
+    // vertices relative to the box's corner (outside the grid too), FP32: small
+    // numbers, error below 1e-6 of the extent
+    const float rx = floorf(xmn - mg), ry = floorf(ymn - mg);
     float x[3], y[3];
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
-        x[m] = (float)(wx[m] - (double)r.i0);
-        y[m] = (float)(wy[m] - (double)r.j0);
+        x[m] = (float)(wx[m] - (double)rx);
+        y[m] = (float)(wy[m] - (double)ry);
     }
     const float ext = fmaxf(fabsf(xmx - xmn), fabsf(ymx - ymn));
     const float area = (x[1] - x[0]) * (y[2] - y[0]) - (y[1] - y[0]) * (x[2] - x[0]);
     // thin (or not a number): the FP64 classification.  The FP32 area's error is
-    // below 1e-6 span^2; the second term is above the needle bound, 1e-9 of the
+    // below 8.4e-7 vs^2; the second term is above the needle bound, 1e-9 of the
     // longest edge times the coordinates
     const float far_ = big + fabsf((float)(g.bb[0] * inv_s)) + fabsf((float)(g.bb[2] * inv_s)) + (float)inv_s;
-    const float span = ext + 2.f + 2.f * mg;          // bounds every coordinate below
-    const bool thick = near_ && fabsf(area) > span * span * 1e-5f + ext * far_ * 4e-9f;
+    const float vs = ext + 2.f + mg;                  // bounds the vertices' coordinates
+    const bool thick = near_ && fabsf(area) > vs * vs * 2e-6f + ext * far_ * 4e-9f;
     const int kind = thick ? kBoxOnly : classify_thin(T);
     if (kind == kPointLike || empty) return kind;
     // error bound of a cross product of FP32 differences: 8.4e-7 span^2, and the
     // columns' own rounding (1e-16 of far_)
+    const float span = ext + 2.f + 3.f * mg;          // bounds the columns' coordinates too
     const float err = 2e-6f * span * span;
     const bool fp32 = near_ && ext < 1e3f && far_ < 1e8f;
     for (int i = r.i0; i <= r.i1; ++i)
@@ -177,7 +180,7 @@ __device__ __forceinline__ int enum_box(const VoxGrid& g, double inv_s, const do
             const bool face = i == 0 || j == 0 || i >= g.Nx - 2 || j >= g.Ny - 2;
             bool in, open = true;
             if (fp32 && !face) {
-                const float px = (float)(i - r.i0), py = (float)(j - r.j0);
+                const float px = (float)i - rx, py = (float)j - ry;
                 const float d1 = (px - x[1]) * (y[0] - y[1]) - (py - y[1]) * (x[0] - x[1]);
                 const float d2 = (px - x[2]) * (y[1] - y[2]) - (py - y[2]) * (x[1] - x[2]);
                 const float d3 = (px - x[0]) * (y[2] - y[0]) - (py - y[0]) * (x[2] - x[0]);

@@ -33,6 +33,13 @@ def soup(rng, kind, n, dims, s, mn):
         z = np.rint(v[:, :1, 2:]) + rng.choice([0.0, 1e-7, -1e-7, 1 + 1e-7, 1.0], (n, 1, 1)) * (L + 0.1) / s * \
             (1 + rng.choice([0, 1e-15, -1e-15, 1e-12, -1e-9, 1e-6], (n, 1, 1)))
         v[:, :, 2:] = z
+    elif kind == "outside":                      # needles and slivers that start far outside and point at the grid
+        d = hi * rng.uniform(0.1, 0.9, (n, 3)) - p[:, 0] * 0
+        a = d + rng.choice([-1, 1], (n, 1)) * rng.uniform(30, 5000, (n, 1)) * rng.normal(size=(n, 3)) * [1, 1, 0.01]
+        far = a + (a - d) * rng.uniform(0.001, 0.2, (n, 1))
+        off = rng.choice([0.0, 1e-11, 1e-8, 1e-5, 0.3], (n, 1)) * rng.normal(size=(n, 3))
+        d = np.where(rng.random((n, 1)) < 0.5, np.rint(d), d)
+        v = np.stack([a, far, np.where(rng.random((n, 1)) < 0.5, d, a + 0.5 * (far - a)) + off], 1)
     elif kind == "far":
         v = p + rng.normal(size=(n, 3, 3)) * rng.choice([1e3, 3e6, 1e9], (n, 1, 1))
     x = v * s + np.array(mn)
@@ -47,15 +54,15 @@ def soup(rng, kind, n, dims, s, mn):
     return t
 
 
-@pytest.mark.parametrize("kind", ["any", "lattice", "needle", "point", "tolerance", "far"])
+@pytest.mark.parametrize("kind", ["any", "lattice", "needle", "point", "tolerance", "far", "outside"])
 @pytest.mark.parametrize("dims,s,mn", [((13, 11, 17), 1.0, (0.0, 0.0, 0.0)), ((9, 14, 70), 0.37, (-175.3, 12.7, 1e4)),
                                        ((12, 7, 33), 0.003, (2.0, -1.0, 0.5)), ((1, 2, 3), 0.25, (0.125, 0.0, -4.0))])
 def test_triangle_soup_matches_oracle(oracle_mod, kind, dims, s, mn):
     O = oracle_mod
-    seed = 1000 * ["any", "lattice", "needle", "point", "tolerance", "far"].index(kind) + dims[0]
+    seed = 1000 * ["any", "lattice", "needle", "point", "tolerance", "far", "outside"].index(kind) + dims[0]
     t = soup(np.random.default_rng(seed), kind, 900, dims, s, mn)
     bb, d = O.explicit_grid((mn, dims), s)
     got = Geometry(t, s, grid=(mn, dims)).flags()
     ref = O.voxelize(t, bb, s, d, binned=False)
     assert np.array_equal(got, ref.reshape(got.shape))
-    assert kind in ("needle", "point") or dims[0] == 1 or 0 < ref.sum() < ref.size
+    assert kind in ("needle", "point", "outside") or dims[0] == 1 or 0 < ref.sum() < ref.size
