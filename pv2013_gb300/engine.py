@@ -17,16 +17,23 @@ from . import _capi
 from ._capi import check, load
 
 
+class _LibArray:
+    """Memory of the library seen by numpy, freed with the last array on it."""
+
+    def __init__(self, ptr, shape):
+        self._ptr, self._free = C.cast(ptr, C.c_void_p), load().lbm_free
+        self.__array_interface__ = {"shape": shape, "typestr": "<f8", "data": (self._ptr.value, False), "version": 3}
+
+    def __del__(self):
+        self._free(self._ptr)
+
+
 def _tri_array(ptr, n):
-    """Copies a library-owned lbm_tri[n] into an (n, 12) float64 array and frees it."""
-    lib = load()
-    try:
-        if n == 0:
-            return np.zeros((0, 12))
-        buf = (C.c_double * (12 * n)).from_address(C.addressof(ptr.contents))
-        return np.frombuffer(buf, dtype=np.float64).reshape(n, 12).copy()
-    finally:
-        lib.lbm_free(C.cast(ptr, C.c_void_p))
+    """A library-owned lbm_tri[n] as an (n, 12) float64 array that owns it."""
+    if n == 0:
+        load().lbm_free(C.cast(ptr, C.c_void_p))
+        return np.zeros((0, 12))
+    return np.asarray(_LibArray(ptr, (n, 12)))
 
 
 def _as_tri_ptr(tris):

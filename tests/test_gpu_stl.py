@@ -102,3 +102,21 @@ def test_large_mesh_timing(tmp_path):
     assert on_device and np.array_equal(host.view(np.uint64), dev.view(np.uint64))
     print(f"\n{len(host)} triangles, {p.stat().st_size / 1e6:.1f} MB: host {t_host * 1e3:.0f} ms, "
           f"device {t_dev * 1e3:.0f} ms")
+
+
+@pytest.mark.parametrize("facets", [1, 1900, 2200, 9000, 30000])
+def test_device_reader_across_read_blocks(tmp_path, facets):
+    """Files below, at and above one block of the readers (0.5 MB), and with more blocks than they hold: the host
+    reader's triangles, line starts and numbers split by a block's end included; a NUL byte in any block is seen."""
+    rng = np.random.default_rng(facets)
+    tris = rng.normal(size=(facets, 12)) * 10.0 ** rng.integers(-3, 4, (facets, 12))
+    path = tmp_path / "f.stl"
+    Reader.writeSTLASCII(path, tris)
+    got, on_device = Reader.readSTLASCIIDevice(path)
+    assert on_device and np.array_equal(got, Reader.readSTLASCII(path)) and got.flags.writeable
+    got[0, 0] = 7.0                                  # the caller's own array
+    text = bytearray(path.read_bytes())
+    text[int(rng.integers(len(text)))] = 0
+    path.write_bytes(text)
+    again, on_device = Reader.readSTLASCIIDevice(path)
+    assert not on_device and np.array_equal(again, Reader.readSTLASCII(path), equal_nan=True)
