@@ -547,8 +547,19 @@ __global__ void __launch_bounds__(256) __maxnreg__((PairMaxReg<Q, S, MODE>::valu
             int32_t zs;
             asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(zs) : "l"(&cw[1].y));     // zslot0, read late
             const int z0 = zs + __popc(zm_all & ((1u << (2 * t)) - 1u));
-            if (zm & 1u) zou_he_half<Q, S>(a, z0, buf, false, step);
-            if (zm & 2u) zou_he_half<Q, S>(a, z0 + (int)(zm & 1u), buf, true, step);
+            if constexpr (Q == 27 && S != ST_F32) {
+                // one copy of the update: D3Q27's faces are long, and a lattice of few
+                // waves waits on their instructions (FP16 AA: 10 240-node pipe 6.9 us a
+                // step with a copy for each half, 6.2 with one, 3.7 M-node ensemble 139
+                // and 133).  FP32 words spill around the loop (198 -> 240), and
+                // D3Q19's routines are short
+#pragma unroll 1
+                for (int h = (zm & 1u) ? 0 : 1; h <= (int)(zm >> 1); ++h)
+                    zou_he_half<Q, S>(a, z0 + (h == 1 ? (int)(zm & 1u) : 0), buf, h == 1, step);
+            } else {
+                if (zm & 1u) zou_he_half<Q, S>(a, z0, buf, false, step);
+                if (zm & 2u) zou_he_half<Q, S>(a, z0 + (int)(zm & 1u), buf, true, step);
+            }
         }
 #pragma unroll
         for (int q = 0; q < Q; ++q) raw[q] = buf[q * 32];
