@@ -117,6 +117,20 @@ struct ListParam {
     int32_t face;      // lbm_face of the LBM_BC_VELOCITY / LBM_BC_PRESSURE kinds
 };
 
+// Everything the paired kernel needs of a Zou-He node in one 64-byte record, in
+// slot order: its profile and its list's parameters (slot, list and amplitude were
+// three dependent loads).
+struct __align__(64) ZNode {
+    double profile;
+    double dir[3];
+    int64_t amp_off;
+    uint32_t amp_len;
+    float rho;
+    int32_t kind, face;
+    int32_t pad[2];
+};
+static_assert(sizeof(ZNode) == 64, "one record, two sectors");
+
 // Per-instance parameters.
 struct InstParam {
     double omega;      // 1/tau
@@ -144,6 +158,7 @@ struct StepArgs {
     void* dst;                // populations written (pull) / same as src (AA)
     int64_t stride;           // elements between population planes (SoA)
     const ZSlot* zslots;
+    const ZNode* znodes;      // paired kernel
     const ListParam* lists;
     const InstParam* insts;
     const double* amp;        // concatenated amplitude tables

@@ -626,6 +626,7 @@ struct lbm_sim {
     int64_t nchunks2s[3] = {0, 0, 0};
     int aa_phase = 0;              // AA: launch n is an even (node-local) launch when n + aa_phase is even
     ZSlot* zslots = nullptr;
+    ZNode* znodes = nullptr;       // the paired kernel's records of the same nodes
     ListParam* lists = nullptr;
     InstParam* insts = nullptr;
     double* amp = nullptr;
@@ -888,7 +889,7 @@ lbm_status sim_launch(lbm_sim* S, int mode, bool dry, void* src, void* dst, int6
     StepArgs a{};
     a.chunks = S->chunks; a.nchunks = S->nchunks;
     a.src = src; a.dst = dst; a.stride = S->stride;
-    a.zslots = S->zslots; a.lists = S->lists; a.insts = S->insts; a.amp = S->amp;
+    a.zslots = S->zslots; a.znodes = S->znodes; a.lists = S->lists; a.insts = S->insts; a.amp = S->amp;
     a.step = step; a.step_base = step_base;
     a.out_f = of; a.out_rho = orho; a.out_u = ou; a.out_pos = S->out_pos; a.n_nodes = S->NF;
     a.mmask = S->mmask;
@@ -1231,6 +1232,15 @@ lbm_status sim_create(const lbm_geometry* const* g, const lbm_sim_params* p, siz
         }
     }
     amp.insert(amp.begin(), 1.0);
+    std::vector<ZNode> znodes(S->store != ST_F64 ? zall.size() : 0);
+    for (size_t i = 0; i < znodes.size(); ++i) {
+        const ListParam& L = lists[(size_t)zall[i].list];
+        znodes[i] = {zall[i].profile, {L.dir[0], L.dir[1], L.dir[2]}, L.amp_off, (uint32_t)L.amp_len, (float)L.rho,
+                     zall[i].kind, L.face, {0, 0}};
+    }
+    LBM_CUDA(cudaMalloc(&S->znodes, sizeof(ZNode) * std::max<size_t>(znodes.size(), 1)));
+    if (!znodes.empty())
+        LBM_CUDA(cudaMemcpyAsync(S->znodes, znodes.data(), sizeof(ZNode) * znodes.size(), cudaMemcpyHostToDevice, st));
     LBM_CUDA(cudaMalloc(&S->lists, sizeof(ListParam) * lists.size()));
     LBM_CUDA(cudaMemcpyAsync(S->lists, lists.data(), sizeof(ListParam) * lists.size(), cudaMemcpyHostToDevice, st));
     LBM_CUDA(cudaMalloc(&S->amp, sizeof(double) * amp.size()));
@@ -2082,6 +2092,7 @@ void lbm_sim_destroy(lbm_sim* S) {
     for (uint2* c : S->even2s) if (c) cudaFree(c);
     if (S->wall_pos) cudaFree(S->wall_pos);
     if (S->zslots) cudaFree(S->zslots);
+    if (S->znodes) cudaFree(S->znodes);
     if (S->lists) cudaFree(S->lists);
     if (S->insts) cudaFree(S->insts);
     if (S->amp) cudaFree(S->amp);

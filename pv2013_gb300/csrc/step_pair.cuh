@@ -163,50 +163,44 @@ __device__ __forceinline__ typename PairWord<S>::W init_half(typename PairWord<S
         return w & (hi ? 0x0000ffffu : 0xffff0000u);
     }
 }
+// one stored value <-> working value
 template <int S, int Q>
-__device__ __forceinline__ float half_plain(typename PairWord<S>::W w, bool hi, int q) {
-    float l, h;
-    f2split(unpack<S, Q>(w, q), l, h);
-    return plain<S, Q>(hi ? h : l, q);
+__device__ __forceinline__ float from_store(typename StoreT<S>::T x, int q) {
+    if constexpr (S == ST_F32) return x - (float)Lat<Q>::w(q);
+    else if constexpr (S == ST_F16S) return __half2float(x);
+    else return __bfloat162float(x);
 }
 template <int S, int Q>
-__device__ __forceinline__ typename PairWord<S>::W set_half_plain(typename PairWord<S>::W w, bool hi, float p, int q) {
-    const float v = unplain<S, Q>(p, q);
-    if constexpr (S == ST_F32) {
-        const uint32_t b = __float_as_uint(v + (float)Lat<Q>::w(q));
-        if (hi) w.y = b; else w.x = b;
-        return w;
-    } else {
-        uint32_t b;
-        if constexpr (S == ST_F16S) b = __half_as_ushort(__float2half_rn(v));
-        else b = __bfloat16_as_ushort(__float2bfloat16_rn(v));
-        return hi ? ((w & 0x0000ffffu) | (b << 16)) : ((w & 0xffff0000u) | b);
-    }
+__device__ __forceinline__ typename StoreT<S>::T to_store(float v, int q) {
+    if constexpr (S == ST_F32) return v + (float)Lat<Q>::w(q);
+    else if constexpr (S == ST_F16S) return __float2half_rn(v);
+    else return __float2bfloat16_rn(v);
 }
 
 // Zou-He on one node (half) of the pair words, in FP32 on plain populations;
 // the results are rounded to the storage format before the collision.
 // raw[q * 32] holds population q's word (a warp's words interleaved in
-// shared memory, so the rest of the pair's words need no registers here)
+// shared memory, so the rest of the pair's words need no registers here); the
+// node's values are every other element there, read and written singly
 template <int Q, int S>
 __device__ __forceinline__ void zou_he_half(const StepArgs& a, int slot, typename PairWord<S>::W* raw, bool hi,
                                             int64_t step) {
     using T = float;
-    const ZSlot z = a.zslots[slot];
-    const ListParam lp = a.lists[z.list];
+    const ZNode& z = a.znodes[slot];
     T p[Q];
+    typename StoreT<S>::T* r = reinterpret_cast<typename StoreT<S>::T*>(raw) + (hi ? 1 : 0);
 #pragma unroll
-    for (int q = 0; q < Q; ++q) p[q] = half_plain<S, Q>(raw[q * 32], hi, q);
+    for (int q = 0; q < Q; ++q) p[q] = plain<S, Q>(from_store<S, Q>(r[q * 64], q), q);
     T v[3] = {T(0), T(0), T(0)};
     if (is_velocity_kind(z.kind)) {
         // 32-bit phase: the step count stays below 2^32 (lbm_sim_step checks)
-        const double amp = a.amp[lp.amp_off + (uint32_t)(step - 1) % (uint32_t)lp.amp_len];
+        const double amp = a.amp[z.amp_off + (uint32_t)(step - 1) % z.amp_len];
         const double sc = amp * z.profile;
-        v[0] = T(sc * lp.dir[0]); v[1] = T(sc * lp.dir[1]); v[2] = T(sc * lp.dir[2]);
+        v[0] = T(sc * z.dir[0]); v[1] = T(sc * z.dir[1]); v[2] = T(sc * z.dir[2]);
     }
-    zou_he_apply<Q, T>(p, z.kind, lp.face, v, T(lp.rho));
+    zou_he_apply<Q, T>(p, z.kind, z.face, v, z.rho);
 #pragma unroll
-    for (int q = 0; q < Q; ++q) raw[q * 32] = set_half_plain<S, Q>(raw[q * 32], hi, p[q], q);
+    for (int q = 0; q < Q; ++q) r[q * 64] = to_store<S, Q>(unplain<S, Q>(p[q], q), q);
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -547,19 +541,12 @@ __global__ void __launch_bounds__(256) __maxnreg__((PairMaxReg<Q, S, MODE>::valu
             int32_t zs;
             asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(zs) : "l"(&cw[1].y));     // zslot0, read late
             const int z0 = zs + __popc(zm_all & ((1u << (2 * t)) - 1u));
-            if constexpr (Q == 27 && S != ST_F32) {
-                // one copy of the update: D3Q27's faces are long, and a lattice of few
-                // waves waits on their instructions (FP16 AA: 10 240-node pipe 6.9 us a
-                // step with a copy for each half, 6.2 with one, 3.7 M-node ensemble 139
-                // and 133).  FP32 words spill around the loop (198 -> 240), and
-                // D3Q19's routines are short
-#pragma unroll 1
-                for (int h = (zm & 1u) ? 0 : 1; h <= (int)(zm >> 1); ++h)
-                    zou_he_half<Q, S>(a, z0 + (h == 1 ? (int)(zm & 1u) : 0), buf, h == 1, step);
-            } else {
-                if (zm & 1u) zou_he_half<Q, S>(a, z0, buf, false, step);
-                if (zm & 2u) zou_he_half<Q, S>(a, z0 + (int)(zm & 1u), buf, true, step);
-            }
+            // the lane's first node whichever half it is, so that lanes with one node
+            // each share a pass (with a pass per half and the node's values merged
+            // into the words: 10 240-node pipe, FP16 AA, 5.8 us a step, 4.9 now; 3.7
+            // M-node ensemble 85.7, 84.5; D3Q27 pipe 6.9, 6.2)
+            zou_he_half<Q, S>(a, z0, buf, !(zm & 1u), step);
+            if (zm == 3u) zou_he_half<Q, S>(a, z0 + 1, buf, true, step);
         }
 #pragma unroll
         for (int q = 0; q < Q; ++q) raw[q] = buf[q * 32];
