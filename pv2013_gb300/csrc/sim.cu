@@ -624,6 +624,7 @@ struct lbm_sim {
     uint2* even2 = nullptr;        // the AA even launch's 8-byte records of chunks2 (k_even_desc)
     uint2* even2s[3] = {nullptr, nullptr, nullptr};
     int64_t nchunks2s[3] = {0, 0, 0};
+    int64_t l2_bytes = 0;          // the device's L2
     int aa_phase = 0;              // AA: launch n is an even (node-local) launch when n + aa_phase is even
     ZSlot* zslots = nullptr;
     ZNode* znodes = nullptr;       // the paired kernel's records of the same nodes
@@ -901,6 +902,7 @@ lbm_status sim_launch(lbm_sim* S, int mode, bool dry, void* src, void* dst, int6
         a.chunks = mode == MODE_AA_ODD ? S->chunks2g : S->chunks2;
         a.nchunks = S->nchunks2;
         a.even_desc = S->even2;
+        a.pf_ahead = S->stride * S->Q * store_bytes(S->store) * (mode == MODE_PULL ? 2 : 1) > S->l2_bytes ? 1 : 0;
         switch (S->store) {
             case ST_F32: return launch_pair_f32(S->Q, mode, S->ra, a, S->wpb, st);
             case ST_F16S: return launch_pair_f16s(S->Q, mode, S->ra, a, S->wpb, st);
@@ -1047,6 +1049,9 @@ void free_graph(lbm_sim* S) {
 lbm_status sim_create(const lbm_geometry* const* g, const lbm_sim_params* p, size_t n, cudaStream_t st, lbm_sim** out) {
     std::unique_ptr<lbm_sim, void (*)(lbm_sim*)> S(new lbm_sim(), lbm_sim_destroy);
     cudaGetDevice(&S->dev);
+    int l2 = 0;
+    LBM_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, S->dev));
+    S->l2_bytes = l2;
     const lbm_sim_params& p0 = p[0];
     if (p0.Q != 19 && p0.Q != 27) return fail(LBM_ERR_ARG, "Q must be 19 or 27 (got %d)", p0.Q);
     S->Q = p0.Q;

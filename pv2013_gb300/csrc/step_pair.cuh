@@ -640,8 +640,13 @@ static lbm_status launch_pair_one(const StepArgs& a, int wpb, cudaStream_t st) {
     // tree's step measured 2.7 % faster; one or two waves ahead: no gain);
     // it prefetches the descriptor one wave ahead (+1 %; half a wave and two
     // waves measured the same within 0.3 %)
+    // Populations that stay in L2 from step to step (a.pf_ahead 0) are not
+    // prefetched: 983 733-node bifurcation, FP16 AA 19.3 us a step with, 19.0
+    // without, D3Q27 29.6 and 29.1, FP32 AA (87 MB) 24.8 and 24.3; FP32 pull (175
+    // MB) 40.1 and 42.2, 3.7 M-node ensemble (155 MB) 84.2 and 87.2
     StepArgs b = a;
-    b.pf_ahead = (int64_t)resident[dev][wpb] * per_block / (MODE == MODE_AA_ODD ? 1 : 2);
+    b.pf_ahead = MODE == MODE_AA_ODD ? (int64_t)resident[dev][wpb] * per_block
+                                     : (a.pf_ahead ? (int64_t)resident[dev][wpb] * per_block / 2 : 0);
     const unsigned grid = (unsigned)(blocks > 0 ? blocks : 1);
     if (a.step_base || blocks > resident[dev][wpb]) {
         k_step2<Q, S, MODE, RA, false><<<grid, 32 * wpb, smem, st>>>(b);
