@@ -673,10 +673,18 @@ static lbm_status geometry_build(lbm_geometry* G, const lbm_tri* tris, size_t nt
     k_boundary<<<g_blocks_for(nwords, 256), 256, 0, st>>>(g, fluid.p, isb.p);
     LBM_TRY(scan::bit_ranks(fluid.p, nwords, nullptr, &G->n_fluid, st));
     LBM_TRY(scan::bit_ranks(isb.p, nwords, rank.p, &G->n_boundary, st));
-    if (G->n_boundary > INT32_MAX) return fail(LBM_ERR_ARG, "more than 2^31 boundary points");
     int64_t* bidx = nullptr;
-    LBM_TRY(dev_alloc(reinterpret_cast<void**>(&bidx), sizeof(int64_t) * std::max<int64_t>(G->n_boundary, 1), st, "boundary points"));
-    k_bit_points<<<g_blocks_for(nwords, 256), 256, 0, st>>>(isb.p, rank.p, nwords, W, g.Nz, bidx);
+    if (G->n_boundary <= (int64_t)UINT32_MAX) {
+        LBM_TRY(dev_alloc(reinterpret_cast<void**>(&bidx), sizeof(int64_t) * std::max<int64_t>(G->n_boundary, 1), st, "boundary points"));
+        k_bit_points<<<g_blocks_for(nwords, 256), 256, 0, st>>>(isb.p, rank.p, nwords, W, g.Nz, bidx);
+    } else {
+        // the ranks are 32-bit: beyond them one byte a point and the 64-bit compaction
+        const int64_t npts = ncol * g.Nz;
+        DBuf<uint8_t> bytes;
+        LBM_TRY(bytes.alloc(npts, "boundary flags", st));
+        k_bit_bytes<<<g_blocks_for(npts, 256), 256, 0, st>>>(isb.p, 0, npts, W, g.Nz, bytes.p);
+        LBM_TRY(scan::compact(bytes.p, npts, &bidx, &G->n_boundary, st));
+    }
     G->d_bidx = bidx;
     DBuf<uint64_t> bmask;
     LBM_TRY(bmask.alloc(G->n_boundary, "boundary masks", st));
