@@ -6,10 +6,41 @@
 
 #include "device.cuh"
 #include "internal.h"
+#include "launch_plan.h"
 
 namespace lbm {
 
 struct Partials;
+
+// LaunchPlans::blocks for kernel `k` on the current device; `twin` (or null) is
+// launched by the same plans.  Fails where no block fits on an SM.
+inline lbm_status resident_blocks(LaunchPlans& plans, const void* k, const void* twin, int wpb, size_t smem, int* blocks) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess || dev < 0 || dev >= LaunchPlans::kDevices)
+        return fail(LBM_ERR_CUDA, "step kernel: device %d not supported", dev);
+    const int n = plans.blocks(
+        dev, wpb, smem,
+        [&](size_t bytes) {
+            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            if (e == cudaSuccess && twin)
+                e = cudaFuncSetAttribute(twin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            return e == cudaSuccess;
+        },
+        [&] {
+            int per_sm = 0, sms = 0;
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * wpb, smem);
+            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            return e == cudaSuccess ? per_sm * sms : 0;
+        });
+    if (n < 1) {
+        cudaGetLastError();
+        return fail(LBM_ERR_CUDA, "step kernel, %d warps a block, %zu B shared: %s", wpb, smem,
+                    e != cudaSuccess ? cudaGetErrorString(e) : "does not fit on an SM");
+    }
+    *blocks = n;
+    return LBM_OK;
+}
 
 lbm_status launch_step_f64(int Q, int mode, bool dry, int ra, const StepArgs& a, const Partials& p, int wpb,
                            cudaStream_t st);

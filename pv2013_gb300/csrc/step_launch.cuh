@@ -29,25 +29,14 @@ static void launch_mode(int mode, bool dry, const StepArgs& a, const Partials& p
 
 template <int Q, int S, int MODE, int RA>
 static lbm_status launch_tma_one(const StepArgs& a, int32_t* err, int wpb, cudaStream_t st) {
-    // one launch configuration per instantiation and block size: the grid is
-    // the number of co-resident blocks (each warp loops over its chunks)
-    static int cached_wpb = 0, cached_blocks = 0;
+    // the grid is at most the co-resident blocks (each warp loops over its chunks)
+    static LaunchPlans plans;
     const size_t smem = (size_t)wpb * stage_count<S>() * StageLayout<Q, S>::BYTES;
-    if (cached_wpb != wpb) {
-        cudaError_t e = cudaFuncSetAttribute(k_step_tma<Q, S, MODE, RA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "step kernel shared memory: %s", cudaGetErrorString(e));
-        int per_sm = 0, dev = 0, sms = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step_tma<Q, S, MODE, RA>, 32 * wpb, smem);
-        if (e == cudaSuccess) e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "occupancy query: %s", cudaGetErrorString(e));
-        if (per_sm < 1) return fail(LBM_ERR_CUDA, "step kernel does not fit on an SM (%zu B shared)", smem);
-        cached_blocks = per_sm * sms;
-        cached_wpb = wpb;
-    }
+    int resident = 0;
+    const lbm_status s = resident_blocks(plans, (const void*)k_step_tma<Q, S, MODE, RA>, nullptr, wpb, smem, &resident);
+    if (s != LBM_OK) return s;
     const int64_t need = (a.nchunks + wpb - 1) / wpb;
-    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(cached_blocks, need));
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(resident, need));
     k_step_tma<Q, S, MODE, RA><<<blocks, 32 * wpb, smem, st>>>(a, err);
     return LBM_OK;
 }

@@ -606,35 +606,16 @@ __global__ void __launch_bounds__(256) __maxnreg__((PairMaxReg<Q, S, MODE>::valu
 template <int Q, int S, int MODE, int RA>
 static lbm_status launch_pair_one(const StepArgs& a, int wpb, cudaStream_t st) {
     // dynamic shared memory: one word per population and lane of each warp
-    // (the Zou-He path); above 48 KB it needs the opt-in attribute
-    // per-device caches (written with the same value by any thread that
-    // fills them): the shared-memory opt-in and the blocks resident at once
-    constexpr int kDevs = 16;
-    static int opted[kDevs] = {0};
-    static int resident[kDevs][9] = {{0}};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevs)
-        return fail(LBM_ERR_CUDA, "paired step kernel: device %d not supported", dev);
+    // (the Zou-He path)
+    static LaunchPlans plans;
     const size_t smem = (size_t)wpb * (Q * 32 * sizeof(typename PairWord<S>::W) + (MODE == MODE_AA_ODD ? 256 : 0));
-    if (smem > 48 * 1024 && opted[dev] < (int)smem) {
-        cudaError_t e = cudaFuncSetAttribute(k_step2<Q, S, MODE, RA, false>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_step2<Q, S, MODE, RA, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "paired step kernel shared memory: %s", cudaGetErrorString(e));
-        opted[dev] = (int)smem;
-    }
+    int resident = 0;                       // blocks at once
+    const lbm_status s = resident_blocks(plans, (const void*)k_step2<Q, S, MODE, RA, false>,
+                                         (const void*)k_step2<Q, S, MODE, RA, true>, wpb, smem, &resident);
+    if (s != LBM_OK) return s;
     const int64_t per_block = (int64_t)wpb << (5 - a.piece_lg);
     const int64_t blocks = (a.nchunks + per_block - 1) / per_block;
-    // prefetch distance: in pieces, from the blocks resident at once
-    if (resident[dev][wpb] == 0) {
-        int sms = 0, nb = 0;
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_step2<Q, S, MODE, RA, false>, 32 * wpb, smem) != cudaSuccess)
-            return fail(LBM_ERR_CUDA, "paired step kernel occupancy: %s", cudaGetErrorString(cudaGetLastError()));
-        resident[dev][wpb] = sms * (nb > 0 ? nb : 1);
-    }
-    // half a wave ahead: measured 0.4 % faster than one wave, 1.5 % faster
+    // prefetch distance, in pieces: half a wave ahead: measured 0.4 % faster than one wave, 1.5 % faster
     // than 1.5 waves.  The AA odd launch prefetches no population window: on
     // its grouped piece table that cost more than it saved (without it the
     // tree's step measured 2.7 % faster; one or two waves ahead: no gain);
@@ -645,10 +626,10 @@ static lbm_status launch_pair_one(const StepArgs& a, int wpb, cudaStream_t st) {
     // without, D3Q27 29.6 and 29.1, FP32 AA (87 MB) 24.8 and 24.3; FP32 pull (175
     // MB) 40.1 and 42.2, 3.7 M-node ensemble (155 MB) 84.2 and 87.2
     StepArgs b = a;
-    b.pf_ahead = MODE == MODE_AA_ODD ? (int64_t)resident[dev][wpb] * per_block
-                                     : (a.pf_ahead ? (int64_t)resident[dev][wpb] * per_block / 2 : 0);
+    b.pf_ahead = MODE == MODE_AA_ODD ? (int64_t)resident * per_block
+                                     : (a.pf_ahead ? (int64_t)resident * per_block / 2 : 0);
     const unsigned grid = (unsigned)(blocks > 0 ? blocks : 1);
-    if (a.step_base || blocks > resident[dev][wpb]) {
+    if (a.step_base || blocks > resident) {
         k_step2<Q, S, MODE, RA, false><<<grid, 32 * wpb, smem, st>>>(b);
         return LBM_OK;
     }
