@@ -964,20 +964,20 @@ void select_piece(lbm_sim* S, int piece) {
 // becomes an AA state, lbm_sim_set_pattern).
 int aa_mode(const lbm_sim* S) { return ((S->steps_done + S->aa_phase) & 1) == 0 ? MODE_AA_EVEN : MODE_AA_ODD; }
 
-// Launches one step at the current state; advances cur/steps_done.
+// Launches one step at the current state and advances cur/steps_done; a launch
+// that failed advances nothing.
 lbm_status sim_one_step(lbm_sim* S, int64_t step_arg, const int64_t* step_base, cudaStream_t st, bool advance_count) {
     Partials np = {nullptr, nullptr, nullptr, nullptr, nullptr};
-    lbm_status s;
     if (S->pattern == LBM_PULL) {
-        s = sim_launch(S, MODE_PULL, false, S->buf[S->cur], S->buf[1 - S->cur], step_arg, step_base, np, nullptr,
-                       nullptr, nullptr, st);
+        LBM_TRY(sim_launch(S, MODE_PULL, false, S->buf[S->cur], S->buf[1 - S->cur], step_arg, step_base, np, nullptr,
+                           nullptr, nullptr, st));
         S->cur = 1 - S->cur;
     } else {
-        s = sim_launch(S, aa_mode(S), false, S->buf[0], S->buf[0], step_arg, step_base, np, nullptr, nullptr, nullptr,
-                       st);
+        LBM_TRY(sim_launch(S, aa_mode(S), false, S->buf[0], S->buf[0], step_arg, step_base, np, nullptr, nullptr,
+                           nullptr, st));
     }
     if (advance_count) S->steps_done++;
-    return s;
+    return LBM_OK;
 }
 
 // Dry launch at the current state (fields and/or monitor partials).
