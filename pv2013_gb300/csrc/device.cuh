@@ -177,6 +177,7 @@ struct StepArgs {
     const uint2* even_desc;   // paired kernel, AA even launch: per piece (n0, len_inst | 64 if a Zou-He lane)
     uint32_t spin_limit;      // TMA-staged kernel: polls of a stage's mbarrier before giving up (0 = default)
     int32_t stall_first;      // TMA-staged kernel, failure tests: each warp's first stage is never issued
+    int32_t chain;            // paired kernel's launcher: the launch may chain to the one before (k_step2, CHAIN)
 };
 
 }  // namespace lbm

@@ -653,6 +653,7 @@ struct lbm_sim {
     double div_tol = 1e-2;
     uint32_t spin_limit = 0;       // TMA-staged kernel's wait limit (0 = its default)
     int32_t stall_first = 0;       // failure tests: the TMA-staged kernel's first stages are not issued
+    bool chain = true;             // direct paired launches may chain (set by lbm_sim_step)
     // wall nodes: output positions in wall-list order (built on first use)
     int64_t* wall_pos = nullptr;
     int64_t nwall = -1;
@@ -897,6 +898,7 @@ lbm_status sim_launch(lbm_sim* S, int mode, bool dry, void* src, void* dst, int6
     a.corr = S->corr;
     a.spin_limit = S->spin_limit;
     a.stall_first = S->stall_first;
+    a.chain = S->chain && !step_base;
     a.piece_lg = S->piece == 8 ? 2 : (S->piece == 16 ? 3 : 4);
     if (!dry && S->npl == 2) {
         a.chunks = mode == MODE_AA_ODD ? S->chunks2g : S->chunks2;
@@ -1461,6 +1463,11 @@ lbm_status lbm_sim_step(lbm_sim* S, int64_t nsteps, uint32_t flags, void* stream
         return fail(LBM_ERR_ARG, "lbm_sim_step: a simulation is limited to 2^32 - 1 steps");
     clear_error();
     cudaStream_t st = (cudaStream_t)stream;
+    // a captured launch becomes a graph node: no programmatic edges there, which not
+    // every user of a graph can read (a stream that cannot be asked is not chained either)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+    S->chain = cap == cudaStreamCaptureStatusNone;
     int64_t left = nsteps;
     const int64_t G = (flags & LBM_STEP_GRAPH) ? graph_length(S, nsteps) : 0;
     if (G) {

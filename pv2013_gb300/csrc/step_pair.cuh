@@ -303,7 +303,8 @@ template <int Q, int S, int MODE> struct PairMaxReg {
 // a step; 10 240-node pipe 7.2 -> 5.7 us).  Graph replay has shorter gaps (the
 // vessel 7.9 us without, 8.5 with), and on larger lattices the wait costs
 // registers and scheduling freedom (vascular tree: 191 -> 205 us), so those
-// launches take the kernel without it.
+// launches take the kernel without it; so do launches into a caller's capture,
+// whose graph then has full dependencies only.
 template <int Q, int S, int MODE, int RA, bool CHAIN>
 __global__ void __launch_bounds__(256) __maxnreg__((PairMaxReg<Q, S, MODE>::value)) k_step2(StepArgs a) {
     using L = Lat<Q>;
@@ -629,7 +630,7 @@ static lbm_status launch_pair_one(const StepArgs& a, int wpb, cudaStream_t st) {
     b.pf_ahead = MODE == MODE_AA_ODD ? (int64_t)resident * per_block
                                      : (a.pf_ahead ? (int64_t)resident * per_block / 2 : 0);
     const unsigned grid = (unsigned)(blocks > 0 ? blocks : 1);
-    if (a.step_base || blocks > resident) {
+    if (!a.chain || blocks > resident) {
         k_step2<Q, S, MODE, RA, false><<<grid, 32 * wpb, smem, st>>>(b);
         return LBM_OK;
     }
