@@ -14,6 +14,13 @@ namespace lbm {
 
 __host__ __device__ constexpr int words_for(int n) { return (n + 31) >> 5; }
 
+// Value of grid point p (x-major, columns of Nz points) in bits of W words a column.
+__host__ __device__ __forceinline__ uint8_t point_bit(const uint32_t* bits, int64_t p, int W, int Nz) {
+    const int64_t col = p / Nz;
+    const int k = (int)(p - col * Nz);
+    return (uint8_t)((bits[col * W + (k >> 5)] >> (k & 31)) & 1u);
+}
+
 // 32x32 bits per warp: lane l gives row l, receives column l
 __device__ __forceinline__ uint32_t transpose32(uint32_t v) {
     const int lane = threadIdx.x & 31;

@@ -470,11 +470,8 @@ __global__ void k_bit_points(const uint32_t* __restrict__ bits, const uint32_t* 
 
 // bytes of grid points [first, first + n)
 __global__ void k_bit_bytes(const uint32_t* __restrict__ bits, int64_t first, int64_t n, int W, int Nz, uint8_t* __restrict__ out) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t p = first + i, col = p / Nz;
-        const int k = (int)(p - col * Nz);
-        out[i] = (uint8_t)((bits[col * W + (k >> 5)] >> (k & 31)) & 1u);
-    }
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = point_bit(bits, first + i, W, Nz);
 }
 
 struct DevPred {
@@ -796,18 +793,37 @@ lbm_status lbm_geometry_info_get(const lbm_geometry* G, lbm_geometry_info* info)
 
 lbm_status lbm_geometry_flags(const lbm_geometry* G, uint8_t* host_out, size_t cap) {
     if (!G || !host_out) return fail(LBM_ERR_ARG, "lbm_geometry_flags: null argument");
+    clear_error();
     size_t n = (size_t)G->grid.Nx * G->grid.Ny * G->grid.Nz;
     if (cap < n) return fail(LBM_ERR_ARG, "lbm_geometry_flags: capacity %zu < %zu", cap, n);
+    const int Nz = G->grid.Nz, W = words_for(Nz);
     // bits to bytes through a scratch of at most 32 MB
     const size_t block = std::min<size_t>(n, size_t(32) << 20);
     cudaStream_t st = 0;
     DBuf<uint8_t> bytes;
-    LBM_TRY(bytes.alloc(block, "node-type bytes", st));
+    if (bytes.alloc(block, "node-type bytes", st) != LBM_OK) {
+        // no room for it: whole columns of bits to the host, about 1 MB at a time
+        clear_error();
+        const int64_t ncol = (int64_t)G->grid.Nx * G->grid.Ny, step = std::max(1, (1 << 18) / W);
+        return guarded("lbm_geometry_flags", [&]() -> lbm_status {
+            std::vector<uint32_t> words((size_t)(std::min(step, ncol) * W));
+            for (int64_t c = 0; c < ncol; c += step) {
+                const int64_t m = std::min(step, ncol - c);
+                LBM_CUDA(cudaMemcpy(words.data(), G->d_fluid + c * W, sizeof(uint32_t) * m * W, cudaMemcpyDeviceToHost));
+                for (int64_t p = 0; p < m * Nz; ++p) host_out[c * Nz + p] = point_bit(words.data(), p, W, Nz);
+            }
+            return LBM_OK;
+        });
+    }
+    // (launched by a call that returns its own status: an error that someone else's
+    // launch left unread is not this call's)
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
     for (size_t at = 0; at < n; at += block) {
         const size_t m = std::min(block, n - at);
-        k_bit_bytes<<<g_blocks_for((int64_t)m, 256), 256, 0, st>>>(G->d_fluid, (int64_t)at, (int64_t)m, words_for(G->grid.Nz),
-                                                                   G->grid.Nz, bytes.p);
-        LBM_CUDA(cudaGetLastError());
+        cfg.gridDim = dim3((unsigned)g_blocks_for((int64_t)m, 256));
+        LBM_CUDA(cudaLaunchKernelEx(&cfg, k_bit_bytes, (const uint32_t*)G->d_fluid, (int64_t)at, (int64_t)m, W, Nz, bytes.p));
         LBM_CUDA(cudaMemcpy(host_out + at, bytes.p, m, cudaMemcpyDeviceToHost));
     }
     return LBM_OK;
