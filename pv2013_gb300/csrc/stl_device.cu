@@ -14,19 +14,16 @@
 // scope, a NUL byte -- makes the reader parse the whole file with the host
 // grammar instead (its recovery rules for broken facets depend on the lines
 // before them), and *on_device reports which path produced the result.
-#include <algorithm>
-#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <thread>
-#include <vector>
 
 #include <fcntl.h>
 #include <unistd.h>
 
 #include <cuda_runtime.h>
 
+#include "block_reader.h"
 #include "device.cuh"
 #include "internal.h"
 #include "scan.cuh"
@@ -179,70 +176,48 @@ struct ParseBufs {
     }
 };
 
-// Reads a file of L bytes into the device buffer: up to kReaders threads, each
-// with two pinned blocks, one being filled while the other is copied.  (Pinning a
-// buffer of the file's size, one read and one copy took 8.9 of the 10.2 ms of a
-// 52 MB file; the whole call takes 2.7 ms now.)  *nul: a NUL byte was seen.
-constexpr int kReaders = 4;
-constexpr size_t kReadBlock = size_t(1) << 19;
-
-struct ReadState {
-    std::atomic<int64_t> next{0};
-    std::atomic<int> io{0}, cuda{0}, nul{0};
-};
-
-void read_blocks(int fd, int64_t L, int dev, char* dst, cudaStream_t st, ReadState* R) {
-    char* host[2] = {nullptr, nullptr};
+// block_reader.h to a device buffer: one stream for all readers
+struct DeviceLink {
+    int dev;
+    char* dst;
+    cudaStream_t st;
     cudaEvent_t done[2] = {nullptr, nullptr};
-    cudaError_t e = cudaSetDevice(dev);
-    for (int b = 0; b < 2 && e == cudaSuccess; ++b) {
-        e = cudaMallocHost(&host[b], std::min<size_t>(kReadBlock, (size_t)L));
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&done[b], cudaEventDisableTiming);
+    int open() {
+        cudaError_t e = cudaSetDevice(dev);
+        for (int b = 0; b < 2 && e == cudaSuccess; ++b) e = cudaEventCreateWithFlags(&done[b], cudaEventDisableTiming);
+        return status(e);
     }
-    bool used[2] = {false, false};
-    for (int b = 0; e == cudaSuccess && !R->io && !R->cuda; b ^= 1) {
-        const int64_t off = R->next.fetch_add((int64_t)kReadBlock);
-        if (off >= L) break;
-        const size_t n = (size_t)std::min<int64_t>((int64_t)kReadBlock, L - off);
-        if (used[b] && (e = cudaEventSynchronize(done[b])) != cudaSuccess) break;
-        size_t got = 0;
-        while (got < n) {
-            const ssize_t k = pread(fd, host[b] + got, n - got, (off_t)(off + (int64_t)got));
-            if (k <= 0) break;
-            got += (size_t)k;
-        }
-        if (got != n) { R->io = 1; break; }
-        if (std::memchr(host[b], 0, n)) R->nul = 1;
-        e = cudaMemcpyAsync(dst + off, host[b], n, cudaMemcpyHostToDevice, st);
-        if (e == cudaSuccess) e = cudaEventRecord(done[b], st);
-        used[b] = true;
+    char* pin(size_t n) {
+        void* p = nullptr;
+        return status(cudaMallocHost(&p, n)) == 0 ? (char*)p : nullptr;
     }
-    if (e != cudaSuccess) { R->cuda = (int)e; cudaGetLastError(); }
-    for (int b = 0; b < 2; ++b) {
-        if (used[b] && done[b]) cudaEventSynchronize(done[b]);      // the copy has left the block
-        if (done[b]) cudaEventDestroy(done[b]);
-        if (host[b]) cudaFreeHost(host[b]);
+    void unpin(char* p) { cudaFreeHost(p); }
+    int copy(int64_t at, const char* block, size_t n, int b) {
+        const cudaError_t e = cudaMemcpyAsync(dst + at, block, n, cudaMemcpyHostToDevice, st);
+        return status(e == cudaSuccess ? cudaEventRecord(done[b], st) : e);
     }
-}
+    int wait(int b) { return status(cudaEventSynchronize(done[b])); }
+    void close() {
+        for (cudaEvent_t e : done) if (e) cudaEventDestroy(e);
+    }
+    static int status(cudaError_t e) {
+        if (e != cudaSuccess) cudaGetLastError();
+        return (int)e;
+    }
+};
 
 lbm_status read_to_device(int fd, const char* path, int64_t L, char* dst, cudaStream_t st, bool* nul) {
     ReadState R;
-    int dev = 0;
-    LBM_CUDA(cudaGetDevice(&dev));
-    const int n = (int)std::min<int64_t>(kReaders, (L + (int64_t)kReadBlock - 1) / (int64_t)kReadBlock);
-    std::vector<std::thread> th;
-    th.reserve(kReaders);                  // (no growth with a running thread in it)
-    for (int i = 1; i < n; ++i) {
-        try {
-            th.emplace_back(read_blocks, fd, L, dev, dst, st, &R);
-        } catch (...) {
-            break;                         // fewer readers, the same result
-        }
-    }
-    read_blocks(fd, L, dev, dst, st, &R);
-    for (std::thread& t : th) t.join();
+    DeviceLink link;
+    LBM_CUDA(cudaGetDevice(&link.dev));
+    link.dst = dst;
+    link.st = st;
+    read_file(fd, L, link, &R);
     if (R.io) return fail(LBM_ERR_IO, "short read of %s", path);
-    if (R.cuda) return fail(LBM_ERR_CUDA, "reading %s to the device: %s", path, cudaGetErrorString((cudaError_t)R.cuda.load()));
+    const bool whole = R.done == L;
+    const int e = R.link ? R.link.load() : (whole ? 0 : R.closed.load());
+    if (e) return fail(LBM_ERR_CUDA, "reading %s to the device: %s", path, cudaGetErrorString((cudaError_t)e));
+    if (!whole) return fail(LBM_ERR_NOMEM, "no memory to read %s through", path);
     *nul = R.nul != 0;
     return LBM_OK;
 }
