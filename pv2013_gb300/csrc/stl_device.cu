@@ -206,6 +206,16 @@ struct DeviceLink {
     }
 };
 
+// reads and goes nowhere
+struct NoLink {
+    int open() { return 0; }
+    char* pin(size_t) { return nullptr; }
+    void unpin(char*) {}
+    int copy(int64_t, const char*, size_t, int) { return 0; }
+    int wait(int) { return 0; }
+    void close() {}
+};
+
 lbm_status read_to_device(int fd, const char* path, int64_t L, char* dst, cudaStream_t st, bool* nul) {
     ReadState R;
     DeviceLink link;
@@ -233,9 +243,17 @@ lbm_status parse_on_device(int fd, const char* path, int64_t L, cudaStream_t st,
         *ok = true;
         return LBM_OK;
     }
-    LBM_TRY(dev_alloc((void**)&B.text, (size_t)L, st, "STL text"));
-    LBM_TRY(dev_alloc((void**)&B.status, sizeof(int32_t), st, "STL status"));
-    LBM_TRY(dev_alloc((void**)&B.flags, (size_t)L, st, "STL line flags"));
+    lbm_status room = dev_alloc((void**)&B.text, (size_t)L, st, "STL text");
+    if (room == LBM_OK) room = dev_alloc((void**)&B.status, sizeof(int32_t), st, "STL status");
+    if (room == LBM_OK) room = dev_alloc((void**)&B.flags, (size_t)L, st, "STL line flags");
+    if (room != LBM_OK) {
+        // the host grammar needs no device memory: a file with a NUL byte is its anyway
+        ReadState R;
+        read_file(fd, L, NoLink{}, &R);
+        if (R.done != L || !R.nul) return room;
+        clear_error();
+        return LBM_OK;
+    }
     LBM_CUDA(cudaMemsetAsync(B.status, 0, sizeof(int32_t), st));
     LBM_CUDA(cudaStreamSynchronize(st));    // the readers copy from other threads
     bool nul = false;
