@@ -336,11 +336,15 @@ __device__ __forceinline__ bool crosses(const VoxGrid& g, double L, const Cand& 
 // and zc - (1 + 1e-7)(L + 0.1).  The computed t and these ends differ from the
 // real ones by less than 32 ulp of (|c/nz| + |qz| + |bb| + L) in z: where that is
 // below 1e-3 of a spacing, only a point within 4e-3 spacings of an end needs the
-// exact test, else the caller tests every point (returns false).
+// exact test, else the caller tests every point (returns false).  The 32 ulp hold
+// where no product with nz under- or overflows: nz within 2^+-800 and a spacing below
+// 1e30, whose lengths (within 1.3e11 spacings by the bound above) stay below 1e42.
 __device__ __forceinline__ bool cross_range(const VoxGrid& g, double inv_s, double L, const Cand& cd, int& lo, int& hi) {
     lo = 0;
     hi = -1;
     if (cd.nz == 0.0 && cd.d0 == 0.0) return true;     // den 0: t is not finite, nothing counts
+    const uint32_t en = ((uint32_t)__double2hiint(cd.nz) >> 20) & 0x7ffu;
+    if (en - (1023u - 800u) > 1600u || !(g.spacing < 1e30)) return false;
     const double h = cd.c / cd.nz, zc = cd.qz + h;
     const double slack = 64.0 * 1.2e-16 * (fabs(h) + fabs(cd.qz) + fabs(g.bb[4]) + fabs(g.bb[5]) + L + 1.0);
     if (!(slack < 1e-3 * g.spacing) || cd.d0 != 0.0) return false;   // (NaN too)
