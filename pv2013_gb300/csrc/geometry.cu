@@ -48,6 +48,7 @@
 #include <vector>
 
 #include "bits.cuh"
+#include "column_range.h"
 #include "device.cuh"
 #include "internal.h"
 #include "scan.cuh"
@@ -139,9 +140,9 @@ __device__ __forceinline__ int enum_box(const VoxGrid& g, double inv_s, const do
     const bool near_ = big < 1e6f;                    // (false for NaN)
     if (near_) {
         r.i0 = (int)ceilf(fmaxf(xmn - mg, 0.f));
-        r.i1 = (int)floorf(fminf(xmx + mg, (float)(g.Nx - 1)));
+        r.i1 = last_column(xmx + mg, g.Nx);
         r.j0 = (int)ceilf(fmaxf(ymn - mg, 0.f));
-        r.j1 = (int)floorf(fminf(ymx + mg, (float)(g.Ny - 1)));
+        r.j1 = last_column(ymx + mg, g.Ny);
     } else {                                          // far from the grid: the same in FP64 (NaN: the whole range)
         const double md = 0.01 * inv_s + 1e-3 + (double)big * 1e-12;
         r.i0 = (int)ceil(fmin(fmax(fmin(wx[0], fmin(wx[1], wx[2])) - md, 0.0), (double)g.Nx));
