@@ -299,8 +299,10 @@ lbm_status lbm_sim_info_get(const lbm_sim* s, lbm_sim_info* info);
  * warps per block, in the current streaming pattern and in the other one
  * where the state converts now (lbm_sim_set_pattern) and its memory fits --
  * for `launches` launches on scratch copies of the state (the simulation does
- * not advance), and keeps the fastest for later steps (converting the state
- * when the pattern changes; results are unchanged).  The layout (structure
+ * not advance), with the kernels of graph replay (LBM_STEP_GRAPH; the choice
+ * is for that mode: direct steps of small lattices chain their launches), and
+ * keeps the fastest for later steps (converting the state when the pattern
+ * changes; results are unchanged).  The layout (structure
  * of arrays) is not a candidate: a blocked layout measured 6 % slower.
  * entries (may be NULL) receives up to cap results, *n (may be NULL) their
  * number.  Needs device memory for one or two more copies of the populations

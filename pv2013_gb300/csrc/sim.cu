@@ -653,7 +653,7 @@ struct lbm_sim {
     double div_tol = 1e-2;
     uint32_t spin_limit = 0;       // TMA-staged kernel's wait limit (0 = its default)
     int32_t stall_first = 0;       // failure tests: the TMA-staged kernel's first stages are not issued
-    bool chain = true;             // direct paired launches may chain (set by lbm_sim_step)
+    bool chain = true;             // direct paired launches may chain (set by lbm_sim_step; the autotuner's do not)
     // wall nodes: output positions in wall-list order (built on first use)
     int64_t* wall_pos = nullptr;
     int64_t nwall = -1;
@@ -1591,6 +1591,10 @@ lbm_status lbm_sim_autotune(lbm_sim* S, int32_t launches, void* stream, lbm_tune
     }
     const int save_pattern = S->pattern, save_npl = S->npl, save_staging = S->staging, save_wpb = S->wpb,
               save_piece = S->piece;
+    // with the kernel that graph replay runs: chained, a candidate that fits one wave
+    // would be timed against others that do not
+    const bool save_chain = S->chain;
+    S->chain = false;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     lbm_status res = LBM_OK;
     auto run = [&](int count) -> lbm_status {
@@ -1629,7 +1633,7 @@ lbm_status lbm_sim_autotune(lbm_sim* S, int32_t launches, void* stream, lbm_tune
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     for (void* b : scratch) if (b) cudaFree(b);
-    S->pattern = save_pattern; S->npl = save_npl; S->staging = save_staging; S->wpb = save_wpb;
+    S->pattern = save_pattern; S->npl = save_npl; S->staging = save_staging; S->wpb = save_wpb; S->chain = save_chain;
     select_piece(S, save_piece);
     if (res != LBM_OK) return res;
     LBM_TRY(check_timeout(S, st));
