@@ -249,21 +249,6 @@ inline lbm_status bit_ranks(const uint32_t* d_in, int64_t n, uint32_t* d_prefix,
     return LBM_OK;
 }
 
-// Counts nonzero entries (synchronises).
-template <class T>
-lbm_status count_nonzero(const T* d_in, int64_t n, int64_t* h_count, cudaStream_t st) {
-    Workspace w;
-    lbm_status s = ws_alloc(w, n, st);
-    if (s != LBM_OK) return s;
-    tile_totals<T><<<(unsigned)w.ntiles, kThreads, 0, st>>>(d_in, n, w.tiles, true);
-    scan_totals<<<1, kThreads, 0, st>>>(w.tiles, w.ntiles, w.total);
-    cudaError_t e = cudaMemcpyAsync(h_count, w.total, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    ws_free(w);
-    if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "count_nonzero: %s", cudaGetErrorString(e));
-    return LBM_OK;
-}
-
 // Ordered indices of nonzero entries into *d_out (allocated here from the
 // stream-ordered pool on st, count in *h_count).
 template <class T>
