@@ -228,7 +228,8 @@ typedef struct lbm_sim_params {
     double tau;                /* relaxation time; omega = 1/tau (Simulation.cpp:11) */
     const lbm_list_bc* bcs;
     size_t nbcs;
-    int32_t warps_per_block;   /* 1..8; 0 = default (4; 1 for nodes_per_lane 2 and small FP64 lattices) */
+    int32_t warps_per_block;   /* 1..8; 0 = default (4; 1 for nodes_per_lane 2 and for FP64 lattices of
+                                  up to 16 chunks an SM) */
     int32_t run_axis;          /* node numbering axis (chunks are runs along it):
                                   1 = y, 2 = z (the reference's x-major order),
                                   0 = the one giving fewer chunks */

@@ -1023,8 +1023,8 @@ lbm_status check_timeout(lbm_sim* S, cudaStream_t st) {
 }
 
 // (the error word comes back with the sums: one copy and one wait a call.  Ten
-// FP32 steps and two monitor calls of a 10 240-node pipe: 166 us with a wait for
-// each and unchained steps, 131 us now)
+// FP32 steps and two monitor calls of a 10 240-node pipe: 147 us with a copy and a
+// wait for the error word, 123 us without)
 lbm_status sim_monitors(lbm_sim* S, lbm_monitors* out, cudaStream_t st) {
     LBM_TRY(sim_dry(S, nullptr, nullptr, nullptr, true, st));
     MonOut h;
@@ -1141,12 +1141,17 @@ lbm_status sim_create(const lbm_geometry* const* g, const lbm_sim_params* p, siz
     S->N = node_off + kLatticeSlack;
     S->NF = out_off;
     S->nchunks = nch;
-    // FP64: a lattice that is one wave of warps (16 an SM) runs in one-warp
-    // blocks, which spread over the SMs to within one chunk (57 821-node vessel:
-    // 38.9 us a step against 42.7 with four-warp blocks); beyond that the
-    // staged ring's warps loop, and four-warp blocks are the better ones
-    // (151 680-node pipe: 92.2 us against 106.6)
-    if (default_wpb && S->store == ST_F64 && nch <= 152 * 16) S->wpb = 1;
+    // FP64: a lattice of up to 16 chunks an SM (one wave of D3Q19 warps; the larger
+    // D3Q27 ring lets 13 on an SM) runs in one-warp blocks, which spread over the SMs
+    // to within one chunk.  us a step, one warp / four warps a block, by chunks:
+    //   D3Q19   416 12.2 / 13.1   896 17.2 / 21.3   1624 28.0 / 29.9   2416 38.8 / 38.9
+    //   D3Q27   416 16.9 / 18.4   896 24.2 / 30.2   1624 39.2 / 41.9   2040 52.5 / 54.6
+    //           2248 57.7 / 55.0 (the one size where it lost)           2416 60.7 / 66.9
+    // Beyond, the warps loop, and where the last round falls decides: D3Q19 2776 45.5 /
+    // 47.5, 5056 86.0 / 82.3; D3Q27 2776 69.5 / 67.7, 9534 234.6 / 210.9.
+    int sms = 0;
+    LBM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, S->dev));
+    if (default_wpb && S->store == ST_F64 && nch <= (int64_t)sms * 16) S->wpb = 1;
     for (int k = 0; k < 3; ++k) S->nchunks2s[k] = nch2[k];
     S->nmask = nmask;
     S->nz = (int64_t)zall.size();
