@@ -177,28 +177,17 @@ __device__ __forceinline__ typename StoreT<S>::T to_store(float v, int q) {
     else return __float2bfloat16_rn(v);
 }
 
-// One stored value in shared memory, inside a word that C++ code writes and reads
-// as a whole: through assembly, which no aliasing rule lets the compiler reorder;
-// asm volatile("" ::: "memory") stands between these and accesses to the words.
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// One stored value inside a word that is stored and loaded as a whole elsewhere:
+// by memcpy, whose bytes alias any type (one 16- or 32-bit access).
 template <int S>
-__device__ __forceinline__ typename StoreT<S>::T ld_elem(uint32_t at) {
-    if constexpr (S == ST_F32) {
-        float v;
-        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at));
-        return v;
-    } else {
-        unsigned short b;
-        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(b) : "r"(at));
-        if constexpr (S == ST_F16S) return __ushort_as_half(b);
-        else return __ushort_as_bfloat16(b);
-    }
+__device__ __forceinline__ typename StoreT<S>::T ld_elem(const char* at) {
+    typename StoreT<S>::T v;
+    __builtin_memcpy(&v, __builtin_assume_aligned(at, sizeof v), sizeof v);
+    return v;
 }
 template <int S>
-__device__ __forceinline__ void st_elem(uint32_t at, typename StoreT<S>::T v) {
-    if constexpr (S == ST_F32) asm volatile("st.shared.f32 [%0], %1;" ::"r"(at), "f"(v));
-    else if constexpr (S == ST_F16S) asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(__half_as_ushort(v)));
-    else asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(__bfloat16_as_ushort(v)));
+__device__ __forceinline__ void st_elem(char* at, typename StoreT<S>::T v) {
+    __builtin_memcpy(__builtin_assume_aligned(at, sizeof v), &v, sizeof v);
 }
 
 // Zou-He on one node (half) of the pair words, in FP32 on plain populations;
@@ -207,13 +196,13 @@ __device__ __forceinline__ void st_elem(uint32_t at, typename StoreT<S>::T v) {
 // shared memory, so the rest of the pair's words need no registers here); the
 // node's values are every other element there, all Q read and written singly
 template <int Q, int S>
-__device__ __forceinline__ void zou_he_half(const StepArgs& a, int slot, const typename PairWord<S>::W* raw, bool hi,
+__device__ __forceinline__ void zou_he_half(const StepArgs& a, int slot, typename PairWord<S>::W* raw, bool hi,
                                             int64_t step) {
     using T = float;
     const ZNode& z = a.znodes[slot];
     T p[Q];
     constexpr uint32_t ES = sizeof(typename StoreT<S>::T);
-    const uint32_t r = smem_u32(raw) + (hi ? ES : 0u);
+    char* r = (char*)raw + (hi ? ES : 0u);
 #pragma unroll
     for (int q = 0; q < Q; ++q) p[q] = plain<S, Q>(from_store<S, Q>(ld_elem<S>(r + q * 64 * ES), q), q);
     T v[3] = {T(0), T(0), T(0)};
@@ -227,6 +216,8 @@ __device__ __forceinline__ void zou_he_half(const StepArgs& a, int slot, const t
 #pragma unroll
     for (int q = 0; q < Q; ++q) st_elem<S>(r + q * 64 * ES, to_store<S, Q>(unplain<S, Q>(p[q], q), q));
 }
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // 0x0000ffff where bit 15 of f is set, | 0xffff0000 where bit 31 is set:
 // prmt with the sign-replicate selector bit (bytes 0-1 from the sign of byte
@@ -561,7 +552,6 @@ __global__ void __launch_bounds__(256) __maxnreg__((PairMaxReg<Q, S, MODE>::valu
         // the warp's words go through shared memory around the per-node update
 #pragma unroll
         for (int q = 0; q < Q; ++q) buf[q * 32] = raw[q];
-        asm volatile("" ::: "memory");
         if (step > 0 && zm) {
             int32_t zs;
             asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(zs) : "l"(&cw[1].y));     // zslot0, read late
@@ -573,7 +563,6 @@ __global__ void __launch_bounds__(256) __maxnreg__((PairMaxReg<Q, S, MODE>::valu
             zou_he_half<Q, S>(a, z0, buf, !(zm & 1u), step);
             if (zm == 3u) zou_he_half<Q, S>(a, z0 + 1, buf, true, step);
         }
-        asm volatile("" ::: "memory");
 #pragma unroll
         for (int q = 0; q < Q; ++q) raw[q] = buf[q * 32];
     }
