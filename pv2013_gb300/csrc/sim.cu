@@ -1470,9 +1470,10 @@ lbm_status lbm_sim_step(lbm_sim* S, int64_t nsteps, uint32_t flags, void* stream
     cudaStream_t st = (cudaStream_t)stream;
     // a captured launch becomes a graph node: no programmatic edges there, which not
     // every user of a graph can read (a stream that cannot be asked is not chained either)
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
-    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
-    S->chain = cap == cudaStreamCaptureStatusNone;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool asked = cudaStreamIsCapturing(st, &cap) == cudaSuccess;
+    if (!asked) cudaGetLastError();
+    S->chain = asked && cap == cudaStreamCaptureStatusNone;
     int64_t left = nsteps;
     const int64_t G = (flags & LBM_STEP_GRAPH) ? graph_length(S, nsteps) : 0;
     if (G) {
