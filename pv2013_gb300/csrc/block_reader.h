@@ -79,7 +79,7 @@ void read_blocks(int fd, int64_t L, Link link, ReadState* R) {
 // every byte has been handed on when R->done is L.
 template <class Link>
 void read_file(int fd, int64_t L, const Link& link, ReadState* R) {
-    const int n = (int)std::min<int64_t>(kReaders, (L + (int64_t)kReadBlock - 1) / (int64_t)kReadBlock);
+    const int n = (int)std::min<int64_t>(kReaders, (L - 1) / (int64_t)kReadBlock + 1);
     std::vector<std::thread> th;
     th.reserve(kReaders);                  // (no growth with a running thread in it)
     for (int i = 1; i < n; ++i) {

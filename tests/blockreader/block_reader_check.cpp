@@ -86,6 +86,17 @@ int main(int argc, char** argv) {
         }
         close(fd);
     }
+    {
+        const size_t size = 0;                               // a directory, of whatever size it claims
+        const int fd = open(argv[1], O_RDONLY);
+        for (int64_t claimed : {int64_t(4096), INT64_MAX}) {
+            Fake f;
+            ReadState R;
+            read_file(fd, claimed, FakeLink{&f}, &R);
+            CHECK(R.io && R.done == 0 && f.copies == 0 && f.pinned == 0);
+        }
+        close(fd);
+    }
     std::printf(bad ? "failed\n" : "block reader ok\n");
     return bad ? 1 : 0;
 }

@@ -26,3 +26,8 @@ def test_files_without_device_memory(tmp_path, engine, facets):
         pytest.skip("the pool's size limit is not enforced")
     assert "LBM_ERR_NOMEM" in str(e.value)
     assert not on_device and np.array_equal(got, Reader.readSTLASCII(nul), equal_nan=True)
+
+
+def test_a_directory_is_refused(tmp_path, engine):
+    with pytest.raises(_capi.LbmError):
+        Reader.readSTLASCIIDevice(tmp_path)
