@@ -25,7 +25,7 @@
 namespace lbm {
 
 // (52 MB file: pinning a buffer of its size, one read and one copy took 8.9 of the
-// reader's 10.2 ms; with blocks the whole call takes 2.7 ms)
+// reader's 10.2 ms; with blocks the whole call takes 2.9 ms)
 constexpr int kReaders = 4;
 constexpr size_t kReadBlock = size_t(1) << 19;
 
